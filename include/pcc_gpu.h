@@ -166,9 +166,9 @@ typedef struct pcc_profile {
   double cell_solves;           /* sum of cell counts over solves */
   long long detect_full_passes; /* detections that rebinned the colony (counted with profiling off too) */
   long long detect_list_passes; /* later ReLCP phases served from the candidate lists */
-  long long bbpgd_grid_launches;  /* BBPGD launches of the multi-block (grid-synchronised) kernel
-                                     (counted with profiling off too) */
-  long long bbpgd_cta_launches;   /* BBPGD launches of the one-block kernels (small colonies) */
+  long long bbpgd_grid_launches;  /* BBPGD launches of more than one block (cluster- or grid-synchronised;
+                                     counted with profiling off too) */
+  long long bbpgd_cta_launches;   /* BBPGD launches of one block (small colonies) */
 } pcc_profile;
 
 typedef struct pcc_ctx pcc_ctx;

@@ -39,28 +39,20 @@ __host__ __device__ inline long long chunk_count(long long m, long long target =
 __host__ __device__ inline long long chunk_lo(long long ch, long long m, long long nchunks) {
   return ch >= nchunks ? m : (ch * m / nchunks) & ~31LL;
 }
-constexpr int kCtaThreads = 4 * kBlock;  // one-CTA form: four 256-thread units
-constexpr int kCtaUnits = kCtaThreads / kBlock;
 constexpr unsigned kFull = 0xffffffffu;
 
 // gamma_k = max(gamma_{k-1} - alpha g_{k-1}, 0): VecWAXPY with PETSc's special
-// cases for the coefficient, then VecPointwiseMax against 0.
+// cases for the coefficient, then VecPointwiseMax against 0.  A coefficient of
+// +-1 needs no case of its own (the product is exact); one of 0 does, for a
+// gradient that is not finite.
 __device__ __forceinline__ double project(double gp, double g, double alpha) {
   const double a = -alpha;
-  double v;
-  if (a == 1.0) v = add(gp, g);
-  else if (a == -1.0) v = sub(gp, g);
-  else if (a == 0.0) v = gp;
-  else v = add(mul(a, g), gp);
+  const double v = a == 0.0 ? gp : add(mul(a, g), gp);
   return v < 0.0 ? 0.0 : v;
 }
 
 // VecScale(x, a) for one entry.
-__device__ __forceinline__ double vscale(double a, double x) {
-  if (a == 1.0) return x;
-  if (a == 0.0) return 0.0;
-  return mul(a, x);
-}
+__device__ __forceinline__ double vscale(double a, double x) { return a == 0.0 ? 0.0 : mul(a, x); }
 
 // Grid barrier of a cooperative launch.  Every block adds one to a
 // monotonic arrival counter; the k-th barrier of the launch is passed once the
@@ -248,16 +240,6 @@ struct GridUnits {  // the multi-block kernel: one unit per block
   __device__ static long long warp() { return ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
   __device__ static long long warps() { return ((long long)gridDim.x * blockDim.x) >> 5; }
 };
-struct CtaUnits {  // the one-CTA kernel: four units in one block, each with its own named barrier
-  static constexpr bool kGrid = false;
-  __device__ static unsigned units() { return kCtaUnits; }
-  __device__ static unsigned unit() { return threadIdx.x / kBlock; }
-  __device__ static int t() { return threadIdx.x % kBlock; }
-  __device__ static void sync() { asm volatile("bar.sync %0, %1;" ::"r"(unit() + 1), "r"(kBlock) : "memory"); }
-  __device__ static long long warp() { return threadIdx.x >> 5; }
-  __device__ static long long warps() { return kCtaThreads / 32; }
-};
-
 // (sum, sum, sum, max) over a warp by an xor tree (every lane ends with the same bits).
 __device__ __forceinline__ void warp_reduce4(double v[4]) {
 #pragma unroll

@@ -67,6 +67,11 @@ long long planar_chunks(size_t m);
 // cooperative kernel, 0 for a one-block launch.
 cudaError_t planar_bbpgd(pcc_ctx* ctx, double dt, bool mixed, const PlanarTrace& tr, int* kind);
 
+// ---- pcc_resident.cu
+// Launches the on-chip BBPGD solve if the constraint set fits it (*taken);
+// full: six D components.  *kind as for planar_bbpgd.
+cudaError_t resident_bbpgd(pcc_ctx* ctx, double dt, bool full, bool mixed, bool* taken, int* kind);
+
 // ---- pcc_update.cu
 cudaError_t reset_ldot(pcc_ctx* ctx);
 cudaError_t grow_cells(pcc_ctx* ctx, double dt);

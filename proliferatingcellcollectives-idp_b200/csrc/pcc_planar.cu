@@ -37,9 +37,10 @@
 // fixed order (in the traced form the last block to arrive does, and
 // publishes the step size and the convergence decision).  The
 // work of a chunk and of a cell never depends on which block does it, so the
-// result does not depend on the grid size: the one-CTA form for small
-// colonies (four 256-thread units in one block, named barriers instead of
-// grid barriers) gives the multi-block kernel's values bit for bit.
+// result does not depend on the grid size.  This kernel streams its operands
+// from memory at every iteration: it takes the constraint sets that are too
+// large for the on-chip kernels (pcc_resident.cu, which give its values bit
+// for bit) and the traced solves.
 //
 // Real = double is the plain FP64 method.  Real = float is the
 // mixed-precision form: D, L, M, U and the D / M products in FP32, while
@@ -55,8 +56,6 @@ namespace pcc {
 
 namespace {
 
-constexpr int kCtaCells = 1024;            // the one-CTA form up to this many cells ...
-constexpr int kCtaConstraints = 4096;      // ... and constraints
 // Co-resident blocks per SM of the multi-block form and the chunk target that
 // goes with it (one chunk per block per iteration), per operand precision.
 template <class Real>
@@ -531,69 +530,6 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
   for (long long c = tid; c < a.m; c += stride) a.phi[c] = ldcg(a.phin + c);
 }
 
-// One-CTA form for colonies of up to kCtaCells cells and kCtaConstraints
-// constraints: the same passes over four units, block barriers instead of
-// grid barriers, unit 0 reducing the chunk partials.  An ordinary launch, so
-// many small colonies' solves run side by side.
-template <class Real>
-__global__ void __launch_bounds__(kCtaThreads, 1) k_bbpgd_planar_cta(PArgs<Real> a) {
-  __shared__ double sm[kCtaUnits][4 * (kBlock / 32)];
-  __shared__ double s_alpha;
-  __shared__ int s_conv;
-  const unsigned unit = CtaUnits::unit();
-  SolverScalars* sc = a.sc;
-
-  cell_pass<Real, CtaUnits, 0>(a, 0, 0.0, false, nullptr, nullptr);
-  __syncthreads();
-  constraint_pass<Real, CtaUnits, 0>(a, 0, 0.0, true, sm[unit], nullptr);
-  __syncthreads();
-  if (unit == 0) {
-    double v[4];
-    reduce_partials<CtaUnits>(a.partials, a.nchunks, v, sm[0]);
-    if (threadIdx.x == 0) {
-      sc->res0 = v[3];
-      sc->residual = v[3];
-      s_alpha = 1.0 / v[3];
-      s_conv = 0;
-    }
-  }
-  __syncthreads();
-
-  long long it = 1;
-  while (it < a.max_it) {
-    const double alpha = s_alpha;
-    const bool check = (it % 10) == 0;
-    cell_pass<Real, CtaUnits, 0>(a, 1, alpha, check, nullptr, nullptr);
-    __syncthreads();
-    constraint_pass<Real, CtaUnits, 0>(a, 1, alpha, check, sm[unit], nullptr);
-    __syncthreads();
-    if (unit == 0) {
-      double v[4];
-      reduce_partials<CtaUnits>(a.partials, a.nchunks, v, sm[0]);
-      if (threadIdx.x == 0) {
-        int conv = 0;
-        if (check) {
-          sc->residual = v[3];
-          if (v[3] <= a.tol) conv = 1;
-        }
-        if (!conv) s_alpha = bb_step(v, it);
-        s_conv = conv;
-        sc->iterations = it;
-      }
-    }
-    __syncthreads();
-    if (s_conv) break;
-    ++it;
-  }
-  if (threadIdx.x == 0) {
-    sc->iterations = it;
-    sc->converged = s_conv;
-    sc->alpha = s_alpha;
-  }
-  if (!s_conv) return;
-  for (long long c = threadIdx.x; c < a.m; c += kCtaThreads) a.phi[c] = a.phin[c];
-}
-
 // ---------------------------------------------------------------- packing
 template <class Real>
 __global__ void k_pack_planar_cons(ConsView cs, long long m, int2* __restrict__ ij,
@@ -724,10 +660,6 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
   a.trace_cap = tr.trace_cap;
   void* args[] = {&a};
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], s);
-  if (!tr.trace && n <= (size_t)kCtaCells && m <= (size_t)kCtaConstraints) {
-    *kind = 0;
-    return cudaLaunchKernel((const void*)k_bbpgd_planar_cta<Real>, dim3(1), dim3(kCtaThreads), args, 0, s);
-  }
   const void* kern = tr.trace ? (const void*)k_bbpgd_planar<Real, 1> : (const void*)k_bbpgd_planar<Real, 0>;
   int& coop = tr.trace ? (sizeof(Real) == 8 ? ctx->coop_planar_tr : ctx->coop_mixed_tr)
                        : (sizeof(Real) == 8 ? ctx->coop_blocks_planar : ctx->coop_blocks_mixed);

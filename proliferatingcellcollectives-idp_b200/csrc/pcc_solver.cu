@@ -607,7 +607,11 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
                       !(ctx->uext_active && !ctx->params.monolayer);
   const bool mixed = planar && ctx->params.precision == PCC_PRECISION_MIXED;
   int kind = 0;
-  if (planar) {  // records ev[0] itself, after packing its operands
+  bool on_chip = false;
+  if (!tracing && (e = resident_bbpgd(ctx, dt, !planar, mixed, &on_chip, &kind))) return e;
+  if (on_chip) {
+    // launched
+  } else if (planar) {  // records ev[0] itself, after packing its operands
     const PlanarTrace tr{trace, ctx->tr_part.p, ctx->trace_dev.p, trace_cap};
     e = planar_bbpgd(ctx, dt, mixed, tr, &kind);
   } else {
