@@ -216,7 +216,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
     if (!vtk_write_trace(ctx->trace_dir, 1, ctx->trace_host))
       return fail(ctx, PCC_ERR_INVALID, "cannot write the BBPGD trace files");
   }
-  CU(grow_cells(ctx, dt), "grow");
+  CU(grow_cells(ctx, dt, !end_check), "grow");
   if (end_check) {
     pcc_status rc = check_device(ctx, "hard step");
     if (rc) return rc;
@@ -246,7 +246,7 @@ pcc_status solve_soft(pcc_ctx* ctx, double dt, pcc_step_stats* st, bool end_chec
   profile_detect(ctx);
   CU(soft_forces_and_move(ctx, dt), "soft");
   ctx->uext_active = false;
-  CU(grow_cells(ctx, dt), "grow");
+  CU(grow_cells(ctx, dt, !end_check), "grow");
   if (end_check) {
     pcc_status rc = check_device(ctx, "soft step");
     if (rc) return rc;
@@ -530,10 +530,7 @@ pcc_status pcc_step(pcc_ctx* ctx, pcc_step_stats* out) {
     return rc;
   }
   ctx->sim_time += dt;
-  if (!ctx->params.fixed_dt) CU(adapt_dt_enqueue(ctx), "adapt_dt");
-  CU(radius_enqueue(ctx), "radius");
-  CU(division_count_enqueue(ctx), "divide");
-  CU(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream), "step");
+  CU(step_end_enqueue(ctx), "step");
   CU(cudaStreamSynchronize(ctx->stream), "step");
   if (ctx->status_host->flags) {
     rc = check_device(ctx, ctx->params.mode == PCC_MODE_SOFT ? "soft step" : "hard step");
@@ -542,13 +539,9 @@ pcc_status pcc_step(pcc_ctx* ctx, pcc_step_stats* out) {
       return rc;
     }
   }
-  if (!ctx->params.fixed_dt) {
-    adapt_dt_collect(ctx);
-    if (ctx->params.dt_cap > 0 && ctx->params.dt > ctx->params.dt_cap) ctx->params.dt = ctx->params.dt_cap;
-  }
-  ctx->radius = radius_collect(ctx);
-  ctx->div_next = (size_t) * reinterpret_cast<int*>(ctx->pinned_ll + kSlotDivs);
-  ctx->div_known = true;
+  step_end_collect(ctx);
+  if (!ctx->params.fixed_dt && ctx->params.dt_cap > 0 && ctx->params.dt > ctx->params.dt_cap)
+    ctx->params.dt = ctx->params.dt_cap;
   ctx->iter++;
   st.n_divided = (long long)added;
   st.dt_used = dt;

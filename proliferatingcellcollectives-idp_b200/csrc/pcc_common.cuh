@@ -31,6 +31,11 @@ struct DevStatus {
   unsigned long long drift_bits;  // largest squared displacement since the lists were built
   unsigned long long lmax_bits;   // longest cell
   unsigned long long maxold_bits; // largest overlap of the constraints of earlier ReLCP phases
+  // end of a step
+  unsigned long long radius_bits;  // colony radius
+  unsigned long long median[2];    // the two middle adaptDt speeds, as ordered keys
+  int divisions;                   // of the next step
+  int pad2;
 };
 
 // Cell arrays (device pointers).

@@ -9,14 +9,14 @@ namespace pcc {
 
 // Slots of ctx->pinned_ll for values copied back at a synchronisation point
 // (slots 0..7 belong to the detection pass).
-constexpr int kSlotMedian = 8;   // two adaptDt median keys
 constexpr int kSlotRadius = 10;  // colony radius bits
 constexpr int kSlotDivs = 11;    // divisions of the next step
 constexpr int kSlotMaxOld = 12;  // largest overlap of the earlier phases' constraints
 
 // ---- pcc_scan_sort.cu
-// out[i] = sum in[0..i-1] for i in [0, n]; out has n+1 entries.
-cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n);
+// out[i] = sum in[0..i-1] for i in [0, n]; out has n+1 entries.  The sum of
+// all goes to *total too (a device address) if given.
+cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total = nullptr);
 // Stable ascending sort of (keys, vals) by the low `bits` bits of keys;
 // keys/vals are sorted in place (scratch from ctx).
 cudaError_t radix_sort_pairs(pcc_ctx* ctx, unsigned long long* keys, int* vals, size_t n, int bits);
@@ -74,21 +74,22 @@ cudaError_t resident_bbpgd(pcc_ctx* ctx, double dt, bool full, bool mixed, bool*
 
 // ---- pcc_update.cu
 cudaError_t reset_ldot(pcc_ctx* ctx);
-cudaError_t grow_cells(pcc_ctx* ctx, double dt);
+// Growth; with step_end also the colony radius and the division flags of the
+// next step (read by step_end_collect after the caller's synchronisation).
+cudaError_t grow_cells(pcc_ctx* ctx, double dt, bool step_end);
 // Division of every cell with len >= 2 l0, daughters appended; returns count.
 // Uses the flags counted at the end of the previous step when ctx->div_known.
 cudaError_t divide_cells(pcc_ctx* ctx, size_t* added);
-// End-of-step work whose results come back in one copy: the division flags
-// and count of the next step, the colony radius, the adaptDt median keys.
-cudaError_t division_count_enqueue(pcc_ctx* ctx);
-cudaError_t radius_enqueue(pcc_ctx* ctx);
-double radius_collect(pcc_ctx* ctx);
-cudaError_t adapt_dt_enqueue(pcc_ctx* ctx);
-void adapt_dt_collect(pcc_ctx* ctx);  // updates ctx->params.dt
+// End of a step: the offsets and the count of the divisions flagged by
+// grow_cells and, unless dt is fixed, the adaptDt median, all into the device
+// status, whose one copy to ctx->status_host is queued; step_end_collect reads
+// it after the caller's synchronisation (radius, divisions of the next step)
+// and adapts ctx->params.dt.
+cudaError_t step_end_enqueue(pcc_ctx* ctx);
+void step_end_collect(pcc_ctx* ctx);
 // Sort cells by x (stable) and renumber.
 cudaError_t sort_cells_by_x(pcc_ctx* ctx);
 cudaError_t colony_radius(pcc_ctx* ctx, double* out);
-cudaError_t adapt_dt(pcc_ctx* ctx);  // updates ctx->params.dt
 cudaError_t mobility(pcc_ctx* ctx);
 
 // ---- pcc_vtk.cu

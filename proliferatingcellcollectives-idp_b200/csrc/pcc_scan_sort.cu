@@ -9,9 +9,13 @@ namespace {
 
 constexpr int kScanItems = 8;                      // items per thread
 constexpr int kScanTile = kBlock * kScanItems;     // 2048 per block
+constexpr int kOneThreads = 1024;                  // one-block scan
+constexpr long long kOneMost = 4LL * kOneThreads * kScanItems;
+constexpr int kSumsMost = 4096;                    // block sums that every block adds up by itself
 
+// Warp-shuffle scan of one value per thread across a block of kThreads.
+template <int kThreads>
 __device__ __forceinline__ int block_exclusive_scan(int v, int* smem, int* total) {
-  // Warp-shuffle scan of one value per thread across a 256-thread block.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int x = v;
 #pragma unroll
@@ -22,19 +26,49 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* smem, int* total
   if (lane == 31) smem[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    int w = lane < (kBlock / 32) ? smem[lane] : 0;
+    int w = lane < (kThreads / 32) ? smem[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       int y = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += y;
     }
-    if (lane < (kBlock / 32)) smem[lane] = w;
+    if (lane < (kThreads / 32)) smem[lane] = w;
   }
   __syncthreads();
   int base = warp ? smem[warp - 1] : 0;
-  *total = smem[kBlock / 32 - 1];
+  *total = smem[kThreads / 32 - 1];
   __syncthreads();
   return base + x - v;
+}
+
+// Scan of a short array by one block: one launch instead of the two below
+// (three before); bound by launch latency.  Up to 32,768 items, four rounds
+// of the block, beyond which the rounds take longer than the second launch.
+__global__ void __launch_bounds__(kOneThreads) k_scan_one(const int* __restrict__ in, int n, int* __restrict__ out,
+                                                          int* __restrict__ total) {
+  __shared__ int sm[kOneThreads / 32];
+  int carry = 0;
+  for (int base = 0; base < n; base += kOneThreads * kScanItems) {
+    const int b = base + (int)threadIdx.x * kScanItems;
+    int v[kScanItems], s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = b + k < n ? in[b + k] : 0;
+      s += v[k];
+    }
+    int tot;
+    int ex = carry + block_exclusive_scan<kOneThreads>(s, sm, &tot);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (b + k < n) out[b + k] = ex;
+      ex += v[k];
+    }
+    carry += tot;
+  }
+  if (threadIdx.x == 0) {
+    out[n] = carry;
+    if (total) *total = carry;
+  }
 }
 
 __global__ void k_scan_reduce(const int* __restrict__ in, size_t n, int* __restrict__ bsum) {
@@ -45,26 +79,36 @@ __global__ void k_scan_reduce(const int* __restrict__ in, size_t n, int* __restr
   for (int k = 0; k < kScanItems; ++k)
     if (base + k < n) s += in[base + k];
   int tot;
-  block_exclusive_scan(s, sm, &tot);
+  block_exclusive_scan<kBlock>(s, sm, &tot);
   if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_blocks(int* bsum, int nb, int* total_out) {
+__global__ void k_scan_blocks(int* bsum, int nb) {
   __shared__ int sm[kBlock / 32];
   int carry = 0;
   for (int base = 0; base < nb; base += kBlock) {
     int i = base + threadIdx.x;
     int v = i < nb ? bsum[i] : 0;
     int tot;
-    int ex = block_exclusive_scan(v, sm, &tot);
+    int ex = block_exclusive_scan<kBlock>(v, sm, &tot);
     if (i < nb) bsum[i] = carry + ex;
     carry += tot;
   }
-  if (threadIdx.x == 0) *total_out = carry;
 }
 
-__global__ void k_scan_apply(const int* __restrict__ in, size_t n, const int* __restrict__ boff, int* __restrict__ out) {
+// scanned: bsum holds the blocks' offsets already (very long arrays);
+// otherwise each block adds up the sums before it.
+__global__ void k_scan_apply(const int* __restrict__ in, size_t n, const int* __restrict__ bsum, bool scanned,
+                             int* __restrict__ out, int* __restrict__ total) {
   __shared__ int sm[kBlock / 32];
+  int before = 0;
+  if (scanned) {
+    before = bsum[blockIdx.x];
+  } else {
+    int s = 0;
+    for (unsigned b = threadIdx.x; b < blockIdx.x; b += kBlock) s += bsum[b];
+    block_exclusive_scan<kBlock>(s, sm, &before);
+  }
   size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   int v[kScanItems];
   int s = 0;
@@ -74,11 +118,15 @@ __global__ void k_scan_apply(const int* __restrict__ in, size_t n, const int* __
     s += v[k];
   }
   int tot;
-  int ex = block_exclusive_scan(s, sm, &tot) + boff[blockIdx.x];
+  int ex = block_exclusive_scan<kBlock>(s, sm, &tot) + before;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     if (base + k < n) out[base + k] = ex;
     ex += v[k];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    out[n] = before + tot;
+    if (total) *total = before + tot;
   }
 }
 
@@ -153,17 +201,22 @@ __global__ void k_radix_scatter(const unsigned long long* __restrict__ keys, con
 
 }  // namespace
 
-cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n) {
+cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total) {
   cudaStream_t s = ctx->stream;
-  size_t nb = (n + kScanTile - 1) / kScanTile;
-  if (nb == 0) nb = 1;
+  if ((long long)n <= kOneMost) {
+    k_scan_one<<<1, kOneThreads, 0, s>>>(in, (int)n, out, total);
+    ctx->launches++;
+    return cudaGetLastError();
+  }
+  const size_t nb = (n + kScanTile - 1) / kScanTile;
   cudaError_t e = ctx->scan_tmp.reserve(nb + 1, 0, s);
   if (e) return e;
   int* bsum = ctx->scan_tmp.p;
+  const bool scanned = nb > (size_t)kSumsMost;
   k_scan_reduce<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum);
-  k_scan_blocks<<<1, kBlock, 0, s>>>(bsum, (int)nb, out + n);
-  k_scan_apply<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum, out);
-  ctx->launches += 3;
+  if (scanned) k_scan_blocks<<<1, kBlock, 0, s>>>(bsum, (int)nb);
+  k_scan_apply<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum, scanned, out, total);
+  ctx->launches += scanned ? 3 : 2;
   return cudaGetLastError();
 }
 

@@ -121,18 +121,7 @@ __global__ void k_divide(CellsView c, long long n, const int* __restrict__ flag,
   }
 }
 
-__global__ void k_x_keys(const double* __restrict__ x, long long n, unsigned long long* __restrict__ keys,
-                         int* __restrict__ vals) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  keys[i] = double_key(x[i]);
-  vals[i] = (int)i;
-}
-
-__global__ void k_gather_cells(CellsView src, CellsView dst, const int* __restrict__ perm, long long n) {
-  long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const int i = perm[j];
+__device__ __forceinline__ void move_cell(const CellsView& src, const CellsView& dst, long long i, long long j) {
   dst.x[j] = src.x[i];
   dst.y[j] = src.y[i];
   dst.z[j] = src.z[i];
@@ -149,48 +138,188 @@ __global__ void k_gather_cells(CellsView src, CellsView dst, const int* __restri
   dst.age[j] = src.age[i];
   dst.ncons[j] = src.ncons[i];
   for (int d = 0; d < 6; ++d) {
-    dst.force[6 * j + d] = src.force[6 * (long long)i + d];
-    dst.vel[6 * j + d] = src.vel[6 * (long long)i + d];
+    dst.force[6 * j + d] = src.force[6 * i + d];
+    dst.vel[6 * j + d] = src.vel[6 * i + d];
   }
 }
 
-__global__ void k_grow(double* __restrict__ len, const double* __restrict__ l0, const double* __restrict__ ldot,
-                       long long n, double dt) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// Ranks by counting, for colonies of up to kRankMost cells: a block takes 32
+// elements, its eight warps an eighth of every tile of keys each, and counts
+// the keys below its own (below or equal among earlier elements: a stable
+// order).  n^2 comparisons, but one launch; an LSD radix sort of the 64-bit
+// keys is 8 x 3 launches whose latency is what a small colony pays for.
+// Measured per x-sort: 225 us in 42 launches (2,474 cells) before.
+constexpr int kRankMost = 16384;
+constexpr int kRankRows = 32;
+constexpr int kRankTile = 2048;
+
+// Rank of element blockIdx.x * 32 + lane among n keys; all threads call, every
+// warp returns it.  key(j) gives the key of element j.
+template <class Key>
+__device__ __forceinline__ int block_rank(int n, Key key, unsigned long long* tile, int* part,
+                                          unsigned long long* own) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int base = (int)blockIdx.x * kRankRows, i = base + lane;
+  const unsigned long long mine = i < n ? key(i) : 0ULL;
+  *own = mine;
+  int count = 0;
+  for (int t0 = 0; t0 < n; t0 += kRankTile) {
+    const int len = n - t0 < kRankTile ? n - t0 : kRankTile;
+    __syncthreads();
+    for (int j = threadIdx.x; j < len; j += kBlock) tile[j] = key(t0 + j);
+    __syncthreads();
+    const int per = (len + 7) / 8, lo = warp * per, hi = lo + per < len ? lo + per : len;
+    // elements before this block's 32, the 32 themselves, elements after
+    const int cut = base - t0 < lo ? lo : base - t0 > hi ? hi : base - t0;
+    const int cut2 = base + kRankRows - t0 < cut ? cut : base + kRankRows - t0 > hi ? hi : base + kRankRows - t0;
+#pragma unroll 8
+    for (int j = lo; j < cut; ++j) count += tile[j] <= mine ? 1 : 0;
+    for (int j = cut; j < cut2; ++j) count += (tile[j] < mine || (tile[j] == mine && t0 + j < i)) ? 1 : 0;
+#pragma unroll 8
+    for (int j = cut2; j < hi; ++j) count += tile[j] < mine ? 1 : 0;
+  }
+  part[warp * 32 + lane] = count;
+  __syncthreads();
+  int rank = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) rank += part[w * 32 + lane];
+  return rank;
+}
+
+// The x-sort of a small colony: ranks, then every warp moves an eighth of the fields.
+__global__ void __launch_bounds__(kBlock) k_rank_sort(CellsView src, CellsView dst, int n) {
+  __shared__ unsigned long long tile[kRankTile];
+  __shared__ int part[kBlock];
+  unsigned long long own;
+  const int j = block_rank(n, [&](int k) { return double_key(src.x[k]); }, tile, part, &own);
+  const int i = (int)blockIdx.x * kRankRows + (int)(threadIdx.x & 31), warp = threadIdx.x >> 5;
   if (i >= n) return;
-  double l = add(len[i], mul(dt, ldot[i]));
-  const double cap = mul(2.0, l0[i]);
-  if (l > cap) l = cap;
-  len[i] = l;
+  const double* from[13] = {src.x, src.y, src.z, src.q0, src.q1, src.q2, src.q3,
+                            src.len, src.l0, src.diam, src.ldot, src.imp, src.stress};
+  double* to[13] = {dst.x, dst.y, dst.z, dst.q0, dst.q1, dst.q2, dst.q3,
+                    dst.len, dst.l0, dst.diam, dst.ldot, dst.imp, dst.stress};
+#pragma unroll
+  for (int f = 0; f < 13; ++f)
+    if ((f & 7) == warp) to[f][j] = from[f][i];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) {
+    if (d == warp) {
+      dst.force[6 * (long long)j + d] = src.force[6 * (long long)i + d];
+      dst.vel[6 * (long long)j + d] = src.vel[6 * (long long)i + d];
+    }
+  }
+  if (warp == 6) dst.age[j] = src.age[i];
+  if (warp == 7) dst.ncons[j] = src.ncons[i];
 }
 
-// max over cells of |x + (len/2 - d/2) t| (spatial/Domain.cpp:148-153)
-__global__ void k_radius(CellsView c, long long n, DevStatus* st) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double m = 0.0;
-  if (i < n) {
-    double t[3];
-    cell_axis(c.q0[i], c.q1[i], c.q2[i], c.q3[i], t);
-    const double half = sub(dvd(c.len[i], 2.0), dvd(c.diam[i], 2.0));
-    const double e[3] = {add(c.x[i], mul(t[0], half)), add(c.y[i], mul(t[1], half)), add(c.z[i], mul(t[2], half))};
-    m = __dsqrt_rn(dot3(e, e));
+// The x-sort of a larger colony: two buckets per cell over [-r, r] in x (r the
+// colony radius; cells beyond it fall in the end buckets), then each cell's
+// rank among its bucket's cells by (key, index).  Buckets hold about half a
+// cell each; a bucket of k cells costs k comparisons for each of them, so a
+// colony standing in one column still sorts, in n^2 / (GPU width).  Five
+// launches where the radix sort of the 64-bit keys took 24.
+struct Buckets {
+  double lo, scale;
+  int count;
+  __device__ __forceinline__ int of(double x) const {
+    const double b = (x - lo) * scale;
+    if (!(b == b)) return (double_key(x) >> 63) ? count - 1 : 0;  // not a number: first or last, as its key sorts
+    return b <= 0.0 ? 0 : b >= (double)(count - 1) ? count - 1 : (int)b;
   }
+};
+
+__global__ void k_bucket_count(const double* __restrict__ x, long long n, Buckets bk, int* __restrict__ cnt,
+                               int* __restrict__ arrival) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) arrival[i] = atomicAdd(&cnt[bk.of(x[i])], 1);
+}
+
+__global__ void k_bucket_place(const double* __restrict__ x, long long n, Buckets bk, const int* __restrict__ off,
+                               const int* __restrict__ arrival, int* __restrict__ cells) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) cells[off[bk.of(x[i])] + arrival[i]] = (int)i;
+}
+
+__global__ void k_bucket_gather(CellsView src, CellsView dst, long long n, Buckets bk, const int* __restrict__ off,
+                                const int* __restrict__ cells) {
+  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  const int i = cells[s];
+  const double x = src.x[i];
+  const unsigned long long mine = double_key(x);
+  const int b = bk.of(x), lo = off[b], hi = off[b + 1];
+  int j = lo;
+  for (int k = lo; k < hi; ++k) {
+    const int o = cells[k];
+    const unsigned long long key = double_key(src.x[o]);
+    j += (key < mine || (key == mine && o < i)) ? 1 : 0;
+  }
+  move_cell(src, dst, i, j);
+}
+
+// Distance of a cell's far end from the origin (spatial/Domain.cpp:148-153).
+__device__ __forceinline__ double end_distance(const CellsView& c, long long i, double len) {
+  double t[3];
+  cell_axis(c.q0[i], c.q1[i], c.q2[i], c.q3[i], t);
+  const double half = sub(dvd(len, 2.0), dvd(c.diam[i], 2.0));
+  const double e[3] = {add(c.x[i], mul(t[0], half)), add(c.y[i], mul(t[1], half)), add(c.z[i], mul(t[2], half))};
+  return __dsqrt_rn(dot3(e, e));
+}
+
+__device__ __forceinline__ void warp_max_into(unsigned long long* dst, double m) {
   for (int o = 16; o > 0; o >>= 1) {
     double w = __shfl_down_sync(0xffffffffu, m, o);
     m = m < w ? w : m;
   }
-  if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(&st->max_bits, (unsigned long long)__double_as_longlong(m));
+  if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(m));
+}
+
+// Growth; at the end of a step (kEnd) also the colony radius and the division
+// flags, which need the grown lengths: one pass over the cells instead of three.
+template <bool kEnd>
+__global__ void k_grow(CellsView c, long long n, double dt, int* __restrict__ flag, DevStatus* st) {
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  double m = 0.0;
+  if (i < n) {
+    double l = add(c.len[i], mul(dt, c.ldot[i]));
+    const double cap = mul(2.0, c.l0[i]);
+    if (l > cap) l = cap;
+    c.len[i] = l;
+    if constexpr (kEnd) {
+      flag[i] = l >= cap ? 1 : 0;
+      m = end_distance(c, i, l);
+    }
+  }
+  if constexpr (kEnd) warp_max_into(&st->radius_bits, m);
+}
+
+__global__ void k_radius(CellsView c, long long n, DevStatus* st) {
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  warp_max_into(&st->max_bits, i < n ? end_distance(c, i, c.len[i]) : 0.0);
 }
 
 // |v| + ldot per cell as an ordered key (Domain::adaptDt, spatial/Domain.cpp:73-77)
+__device__ __forceinline__ unsigned long long speed_key(const CellsView& c, long long i) {
+  const double* v = c.vel + 6 * i;
+  const double vv[3] = {v[0], v[1], v[2]};
+  return double_key(add(__dsqrt_rn(dot3(vv, vv)), c.ldot[i]));
+}
+
 __global__ void k_speed_keys(CellsView c, long long n, unsigned long long* __restrict__ keys, int* __restrict__ vals) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double* v = c.vel + 6 * i;
-  const double vv[3] = {v[0], v[1], v[2]};
-  const double s = add(__dsqrt_rn(dot3(vv, vv)), c.ldot[i]);
-  keys[i] = double_key(s);
+  keys[i] = speed_key(c, i);
   vals[i] = (int)i;
+}
+
+// The keys of ranks lo and lo + 1 of a small colony's speeds.
+__global__ void __launch_bounds__(kBlock) k_rank_median(CellsView c, int n, int lo, DevStatus* st) {
+  __shared__ unsigned long long tile[kRankTile];
+  __shared__ int part[kBlock];
+  unsigned long long own;
+  const int r = block_rank(n, [&](int k) { return speed_key(c, k); }, tile, part, &own);
+  const int i = (int)blockIdx.x * kRankRows + (int)(threadIdx.x & 31);
+  if (threadIdx.x < 32 && i < n && (r == lo || r == lo + 1)) st->median[r - lo] = own;
 }
 
 double key_to_double(unsigned long long k) {
@@ -207,25 +336,20 @@ cudaError_t reset_ldot(pcc_ctx* ctx) {
   return cudaMemsetAsync(ctx->cells.ldot.p, 0, ctx->n * sizeof(double), ctx->stream);
 }
 
-cudaError_t grow_cells(pcc_ctx* ctx, double dt) {
-  if (!ctx->n) return cudaSuccess;
-  k_grow<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(ctx->cells.len.p, ctx->cells.l0.p, ctx->cells.ldot.p,
-                                                       (long long)ctx->n, dt);
-  ctx->launches++;
-  return cudaGetLastError();
-}
-
-cudaError_t division_count_enqueue(pcc_ctx* ctx) {
+cudaError_t grow_cells(pcc_ctx* ctx, double dt, bool step_end) {
   cudaStream_t s = ctx->stream;
   const size_t n = ctx->n;
-  cudaError_t e;
-  if ((e = ctx->div_flag.reserve(n + 1, 0, s)) || (e = ctx->div_off.reserve(n + 1, 0, s))) return e;
-  if (n) {
-    k_div_flag<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.len.p, ctx->cells.l0.p, (long long)n, ctx->div_flag.p);
-    ctx->launches++;
+  if (step_end) cudaMemsetAsync(&ctx->status->radius_bits, 0, sizeof(unsigned long long), s);
+  if (!n) return cudaSuccess;
+  if (step_end) {
+    cudaError_t e;
+    if ((e = ctx->div_flag.reserve(n + 1, 0, s))) return e;
+    k_grow<true><<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), (long long)n, dt, ctx->div_flag.p, ctx->status);
+  } else {
+    k_grow<false><<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), (long long)n, dt, nullptr, ctx->status);
   }
-  if ((e = exclusive_scan(ctx, ctx->div_flag.p, ctx->div_off.p, n))) return e;
-  return cudaMemcpyAsync(ctx->pinned_ll + kSlotDivs, ctx->div_off.p + n, sizeof(int), cudaMemcpyDeviceToHost, s);
+  ctx->launches++;
+  return cudaGetLastError();
 }
 
 cudaError_t divide_cells(pcc_ctx* ctx, size_t* added) {
@@ -238,7 +362,12 @@ cudaError_t divide_cells(pcc_ctx* ctx, size_t* added) {
   if (ctx->div_known) {  // counted at the end of the previous step, on these very cells
     k = ctx->div_next;
   } else {
-    if ((e = division_count_enqueue(ctx))) return e;
+    if ((e = ctx->div_flag.reserve(n + 1, 0, s)) || (e = ctx->div_off.reserve(n + 1, 0, s))) return e;
+    k_div_flag<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.len.p, ctx->cells.l0.p, (long long)n, ctx->div_flag.p);
+    ctx->launches++;
+    if ((e = exclusive_scan(ctx, ctx->div_flag.p, ctx->div_off.p, n))) return e;
+    if ((e = cudaMemcpyAsync(ctx->pinned_ll + kSlotDivs, ctx->div_off.p + n, sizeof(int), cudaMemcpyDeviceToHost, s)))
+      return e;
     if ((e = cudaStreamSynchronize(s))) return e;
     k = (size_t) * reinterpret_cast<int*>(ctx->pinned_ll + kSlotDivs);
   }
@@ -259,66 +388,79 @@ cudaError_t sort_cells_by_x(pcc_ctx* ctx) {
   const size_t n = ctx->n;
   cudaError_t e;
   if (n <= 1) return cudaSuccess;
-  if ((e = ctx->keys.reserve(n, 0, s)) || (e = ctx->perm.reserve(n, 0, s))) return e;
   if ((e = ctx->cells_alt.reserve(n, 0, s))) return e;
-  k_x_keys<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, ctx->keys.p, ctx->perm.p);
-  ctx->launches++;
-  if ((e = radix_sort_pairs(ctx, ctx->keys.p, ctx->perm.p, n, 64))) return e;
-  k_gather_cells<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), ctx->perm.p, (long long)n);
-  ctx->launches++;
+  if (n <= (size_t)kRankMost) {
+    k_rank_sort<<<grid_for((long long)n, kRankRows), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), (int)n);
+    ctx->launches++;
+  } else {
+    const double r = ctx->radius > 0 && std::isfinite(ctx->radius) ? ctx->radius : 1.0;
+    Buckets bk;
+    bk.count = (int)(2 * n);
+    bk.lo = -r;
+    bk.scale = bk.count / (2.0 * r);
+    if ((e = ctx->perm.reserve(n, 0, s)) || (e = ctx->perm_alt.reserve(n, 0, s)) ||
+        (e = ctx->sort_hist.reserve(2 * (size_t)bk.count + 1, 0, s)))
+      return e;
+    int *cnt = ctx->sort_hist.p, *off = cnt + bk.count;
+    cudaMemsetAsync(cnt, 0, bk.count * sizeof(int), s);
+    k_bucket_count<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, cnt, ctx->perm_alt.p);
+    if ((e = exclusive_scan(ctx, cnt, off, bk.count))) return e;
+    k_bucket_place<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, off, ctx->perm_alt.p, ctx->perm.p);
+    k_bucket_gather<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), (long long)n, bk, off,
+                                                  ctx->perm.p);
+    ctx->launches += 3;
+  }
   ctx->cells.swap(ctx->cells_alt);
   return cudaGetLastError();
 }
 
-cudaError_t radius_enqueue(pcc_ctx* ctx) {
+cudaError_t colony_radius(pcc_ctx* ctx, double* out) {
   cudaStream_t s = ctx->stream;
   cudaMemsetAsync(&ctx->status->max_bits, 0, sizeof(unsigned long long), s);
   if (ctx->n) {
     k_radius<<<grid_for(ctx->n), kBlock, 0, s>>>(ctx->cells.view(), (long long)ctx->n, ctx->status);
     ctx->launches++;
   }
-  return cudaMemcpyAsync(ctx->pinned_ll + kSlotRadius, &ctx->status->max_bits, sizeof(unsigned long long),
-                         cudaMemcpyDeviceToHost, s);
-}
-
-double radius_collect(pcc_ctx* ctx) {
-  double r;
-  std::memcpy(&r, ctx->pinned_ll + kSlotRadius, sizeof r);
-  return r;
-}
-
-cudaError_t colony_radius(pcc_ctx* ctx, double* out) {
-  cudaError_t e = radius_enqueue(ctx);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(ctx->pinned_ll + kSlotRadius, &ctx->status->max_bits, sizeof(unsigned long long),
+                                  cudaMemcpyDeviceToHost, s);
+  if (!e) e = cudaStreamSynchronize(s);
   if (e) return e;
-  *out = radius_collect(ctx);
+  std::memcpy(out, ctx->pinned_ll + kSlotRadius, sizeof *out);
   return cudaSuccess;
+}
+
+cudaError_t step_end_enqueue(pcc_ctx* ctx) {
+  cudaStream_t s = ctx->stream;
+  const size_t n = ctx->n;
+  cudaError_t e;
+  if ((e = ctx->div_flag.reserve(n + 1, 0, s)) || (e = ctx->div_off.reserve(n + 1, 0, s))) return e;
+  if ((e = exclusive_scan(ctx, ctx->div_flag.p, ctx->div_off.p, n, &ctx->status->divisions))) return e;
+  if (!ctx->params.fixed_dt && n) {
+    const size_t lo = n % 2 == 0 ? n / 2 - 1 : n / 2;
+    if (n <= (size_t)kRankMost) {
+      k_rank_median<<<grid_for((long long)n, kRankRows), kBlock, 0, s>>>(ctx->cells.view(), (int)n, (int)lo,
+                                                                        ctx->status);
+      ctx->launches++;
+    } else {
+      if ((e = ctx->keys.reserve(n, 0, s)) || (e = ctx->perm.reserve(n, 0, s))) return e;
+      k_speed_keys<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), (long long)n, ctx->keys.p, ctx->perm.p);
+      ctx->launches++;
+      if ((e = radix_sort_pairs(ctx, ctx->keys.p, ctx->perm.p, n, 64))) return e;
+      if ((e = cudaMemcpyAsync(ctx->status->median, ctx->keys.p + lo, 2 * sizeof(unsigned long long),
+                               cudaMemcpyDeviceToDevice, s)))
+        return e;
+    }
+  }
+  return cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
 }
 
 // Domain::adaptDt (spatial/Domain.cpp:69-118): median of |v| + ldot (for an
 // even count, the mean of the two middle values), dt* = cfl*tol/median,
-// dt <- clamp(0.99 dt + 0.01 dt*, 0.9 dt, 1.1 dt).  The enqueue half sorts the
-// speeds on the device and queues the copy of the middle keys; the collect
-// half, after the caller's synchronisation, does the host arithmetic.
-cudaError_t adapt_dt_enqueue(pcc_ctx* ctx) {
-  cudaStream_t s = ctx->stream;
-  const size_t n = ctx->n;
-  cudaError_t e;
-  if (!n) return cudaSuccess;
-  if ((e = ctx->keys.reserve(n, 0, s)) || (e = ctx->perm.reserve(n, 0, s))) return e;
-  k_speed_keys<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), (long long)n, ctx->keys.p, ctx->perm.p);
-  ctx->launches++;
-  if ((e = radix_sort_pairs(ctx, ctx->keys.p, ctx->perm.p, n, 64))) return e;
-  const size_t lo = n % 2 == 0 ? n / 2 - 1 : n / 2;
-  return cudaMemcpyAsync(ctx->pinned_ll + kSlotMedian, ctx->keys.p + lo,
-                         2 * sizeof(unsigned long long) - (n == 1 ? sizeof(unsigned long long) : 0),
-                         cudaMemcpyDeviceToHost, s);
-}
-
-void adapt_dt_collect(pcc_ctx* ctx) {
+// dt <- clamp(0.99 dt + 0.01 dt*, 0.9 dt, 1.1 dt).
+static void adapt_dt(pcc_ctx* ctx) {
   const size_t n = ctx->n;
   if (!n) return;
-  const unsigned long long* pk = reinterpret_cast<const unsigned long long*>(ctx->pinned_ll + kSlotMedian);
+  const unsigned long long* pk = ctx->status_host->median;
   double med;
   if (n % 2 == 0) {
     const double lower = key_to_double(pk[0]), upper = key_to_double(pk[1]);
@@ -339,12 +481,12 @@ void adapt_dt_collect(pcc_ctx* ctx) {
   ctx->params.dt = nd;
 }
 
-cudaError_t adapt_dt(pcc_ctx* ctx) {
-  cudaError_t e = adapt_dt_enqueue(ctx);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
-  if (e) return e;
-  adapt_dt_collect(ctx);
-  return cudaSuccess;
+void step_end_collect(pcc_ctx* ctx) {
+  const DevStatus& st = *ctx->status_host;
+  if (!ctx->params.fixed_dt) adapt_dt(ctx);
+  std::memcpy(&ctx->radius, &st.radius_bits, sizeof ctx->radius);
+  ctx->div_next = (size_t)st.divisions;
+  ctx->div_known = true;
 }
 
 }  // namespace pcc
