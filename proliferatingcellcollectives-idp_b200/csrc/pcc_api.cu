@@ -171,16 +171,17 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
   };
   while ((long long)phase < ctx->params.max_recursive_iterations) {
     const size_t before = ctx->ncons;
-    if (before) CU(max_overlap_enqueue(ctx, 0, before), "max_overlap");
     size_t added = 0;
     double ov_new = 0.0;
     if (ctx->profiling) cudaEventRecord(ctx->ev[2], ctx->stream);
     CU(detect_contacts(ctx, phase == 0 ? .25 : tol, phase, phase > 0, &added, &ov_new), "detect");
-    if (ctx->n == 0) CU(cudaStreamSynchronize(ctx->stream), "detect");  // an empty colony's detection did not wait
+    if (ctx->n == 0) {  // an empty colony's detection did not wait
+      CU(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream), "detect");
+      CU(cudaStreamSynchronize(ctx->stream), "detect");
+    }
     pcc_status rc = collect();  // the previous phase's BBPGD, now complete
     if (rc) return rc;
-    double ov_old = 0.0;
-    if (before) std::memcpy(&ov_old, ctx->pinned_ll + kSlotMaxOld, sizeof ov_old);
+    const double ov_old = before ? ctx->solved_overlap : 0.0;
     max_ov = ov_old < ov_new ? ov_new : ov_old;
     if (max_ov <= tol && phase > 0) {
       profile_detect(ctx);
@@ -205,6 +206,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
     ++phase;
   }
   if (ctx->bbpgd_pending) {  // the loop ran out of phases right after a solve
+    CU(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream), "bbpgd");
     CU(cudaStreamSynchronize(ctx->stream), "bbpgd");
     pcc_status rc = collect();
     if (rc) return rc;
@@ -464,6 +466,8 @@ pcc_status pcc_upload_cells(pcc_ctx* ctx, const pcc_cells* c, size_t n) {
   ctx->div_known = false;
   CU(cudaStreamSynchronize(s), "upload");
   CU(colony_radius(ctx, &ctx->radius), "radius");
+  ctx->box_known = true;
+  ctx->flat = true;
   return PCC_OK;
 }
 

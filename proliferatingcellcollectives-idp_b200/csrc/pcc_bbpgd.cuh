@@ -153,6 +153,17 @@ struct GridBarrier {
   }
 };
 
+// Folds the largest overlap of a thread's returned constraints (max(-phi, 0))
+// into the scalars; all lanes of a warp call.
+__device__ __forceinline__ void fold_overlap(SolverScalars* sc, double v) {
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_down_sync(0xffffffffu, v, o);
+    v = v < w ? w : v;
+  }
+  if ((threadIdx.x & 31) == 0 && v > 0.0) atomicMax(&sc->overlap_bits, (unsigned long long)__double_as_longlong(v));
+}
+__device__ __forceinline__ double overlap_of(double most, double phi) { return most < -phi ? -phi : most; }
+
 __device__ __forceinline__ double proj_grad_abs(double g, double gam) {
   double v = gam > 0 ? g : (g < 0.0 ? g : 0.0);
   return fabs(v);

@@ -6,6 +6,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "pcc_gpu.h"
@@ -25,18 +26,22 @@ enum : unsigned {
 struct DevStatus {
   unsigned flags;
   int where;
+  // contact detection: cleared as one block at the start of a pass
   unsigned long long max_bits;    // running max of a non-negative double (bit pattern)
-  unsigned list_flags;            // contact detection: candidate lists overflowed / stale
-  unsigned pad;
   unsigned long long drift_bits;  // largest squared displacement since the lists were built
   unsigned long long lmax_bits;   // longest cell
-  unsigned long long maxold_bits; // largest overlap of the constraints of earlier ReLCP phases
+  unsigned list_flags;            // candidate lists overflowed / stale, cells outside the assumed box
+  unsigned nonplanar;             // a cell is out of the plane
+  unsigned box_lo[3], box_hi[3];  // bounding box of the bins, as keys whose maximum is taken (box_key)
+  int count;                      // contacts found
+  int pad;
   // end of a step
   unsigned long long radius_bits;  // colony radius
   unsigned long long median[2];    // the two middle adaptDt speeds, as ordered keys
   int divisions;                   // of the next step
   int pad2;
 };
+constexpr size_t kDetectBegin = offsetof(DevStatus, max_bits), kDetectBytes = offsetof(DevStatus, radius_bits) - kDetectBegin;
 
 // Cell arrays (device pointers).
 struct CellsView {

@@ -83,6 +83,7 @@ struct SolverScalars {
   double res0;                   // initial residual
   // cell-unit counters of the multi-block planar cell pass, two sets used by
   // alternate iterations, one counter per 128-byte line; not copied back
+  unsigned long long overlap_bits;  // largest overlap of the constraints after a converged solve
   alignas(128) unsigned long long take[2][kTakeGroups][16];
 };
 constexpr size_t kScalarsCopied = offsetof(SolverScalars, take);
@@ -108,10 +109,11 @@ struct pcc_ctx {
   pcc::ConsBufs cons;
 
   // detection scratch
-  pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_cursor, bin_cells, cand_cnt, cand_off;
+  pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_cursor, bin_raw, bin_cells, cand_cnt, cand_off;
   pcc::DevBuf<double> pk;  // packed per-cell geometry in bin order
   pcc::DevBuf<int> ghost;
-  pcc::DevBuf<int> bbox;   // [6] min/max bin coordinates, [7] non-planar flag
+  bool box_known = false;  // radius bounds the centres of the resident cells
+  bool flat = true;        // no cell left the plane z = 0 since the upload
   // candidate partner lists of the last full neighbourhood pass (list-major)
   pcc::DevBuf<int> plist, plist_n, slot_of;
   pcc::DevBuf<double> xref;  // cell positions when the lists were built
@@ -159,6 +161,7 @@ struct pcc_ctx {
   pcc::SolverScalars* scal_host = nullptr;  // pinned: BBPGD scalars of a launch not yet read
   bool bbpgd_pending = false;               // a BBPGD launch whose scalars are still on their way
   double bbpgd_pending_bytes = 0.0;         // its algorithmic bytes per iteration
+  double solved_overlap = 0.0;              // largest overlap that the last solve left
   bool div_known = false;                   // div_flag / div_off / div_next describe the resident cells
   size_t div_next = 0;                      // divisions the next step commits
 

@@ -6,17 +6,31 @@
 // reference grid (origin -1, edge linked_cell_size, floor), so the candidate
 // pairs -- every unordered pair in the same or an adjacent bin of the
 // 27-stencil -- are the same set.  Binning is a counting sort: atomic counts,
-// an exclusive scan, an atomic scatter and a per-bin sort by id, which makes
-// the bin contents (and everything downstream) deterministic.  Each cell's
-// geometry is packed once per phase in bin order so the neighbour scans read
-// contiguous 32-byte groups.  The full pass scans the stencil once, counts
-// the constraints and records each cell's partners within a wider reach in a
-// candidate list; the emit pass and the later ReLCP phases of the same step
-// walk those lists (with the reference's bin-adjacency test on the current
-// bins and a displacement bound that proves no other pair can qualify).
-// Counts are scanned into offsets, so constraints come out grouped by the
-// smaller id in a fixed order, without atomics on the output.
+// an exclusive scan, an atomic scatter and each cell's rank by id within its
+// bin, which makes the bin contents (and everything downstream)
+// deterministic.  Each cell's geometry is packed once per phase in bin order
+// so the neighbour scans read contiguous 32-byte groups.  The full pass scans
+// the stencil once, counts the constraints and records each cell's partners
+// within a wider reach in a candidate list; the emit pass and the later ReLCP
+// phases of the same step walk those lists (with the reference's bin-adjacency
+// test on the current bins and a displacement bound that proves no other pair
+// can qualify).  Counts are scanned into offsets, so constraints come out
+// grouped by the smaller id in a fixed order, without atomics on the output.
+//
+// The pair passes are chains of dependent loads and of double-precision
+// geometry, so they are bound by latency unless the GPU is full: kPairLanes
+// lanes share a cell's candidates.  Measured (stencil scan / list count / list
+// emit, us, ncu, cold caches): one thread per cell 56 / 23 / 27 at 447 cells
+// and 84 / 35 / 45 at 44,700; eight lanes 13 / 8 / 8 and 57 / 37 / 35; four
+// lanes 62 / 31 / 35 at 44,700.  At 302,180 cells, where memory bounds them,
+// 295 / 128 / 195 with one thread, 319 / 150 / 185 with four lanes and 337 /
+// 245 / 207 with eight.
+//
+// At the end of a pass the host needs the number of contacts and a few flags:
+// they are collected in the device status, cleared by one memset and read by
+// one copy per pass.
 #include <cmath>
+#include <cstring>
 
 #include "pcc_kernels.hpp"
 
@@ -28,7 +42,8 @@ constexpr int kPack = 16;  // doubles per packed cell record
 // record layout: [x y z len | sx sy sz diam | ex ey ez gid | tx ty tz ghost]
 constexpr int kList = 32;  // candidate partners kept per cell
 constexpr double kListReach = 0.25;  // list reach beyond contact: the first ReLCP phase's tolerance
-enum : unsigned { kListOverflow = 1u, kListStale = 2u };
+constexpr int kFewCells = 20000;  // below: 8 lanes per cell in the pair passes, from there on 4
+enum : unsigned { kListOverflow = 1u, kListStale = 2u, kOutOfBox = 4u };
 
 // Warp-wide max of a non-negative double folded into *dst (all lanes call).
 __device__ __forceinline__ void warp_max_into(unsigned long long* dst, double v) {
@@ -39,24 +54,32 @@ __device__ __forceinline__ void warp_max_into(unsigned long long* dst, double v)
   if ((threadIdx.x & 31) == 0 && v > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(v));
 }
 
-// Bins every cell on its centre (origin -1, edge h, floor: the reference
-// grid), decides its self-ghost, and folds the bin bounding box, the
-// planarity flag, the longest cell and (when xref is given) the largest
-// squared displacement since xref into the status, one atomic per warp.
-__global__ void k_bin(CellsView c, size_t n, double h, int ghost_mode, const double* __restrict__ xref,
-                      int* __restrict__ binxyz, int* __restrict__ bbox, int* __restrict__ ghost, DevStatus* st) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = i < n;
-  int bx = 0, by = 0, bz = 0, nonplanar = 0;
+// Bounding-box keys: a maximum that starts from 0 serves for both ends.
+__host__ __device__ inline unsigned box_key_hi(int b) { return (unsigned)b ^ 0x80000000u; }
+__host__ __device__ inline unsigned box_key_lo(int b) { return ~box_key_hi(b); }
+
+struct Grid {
+  int mx, my, mz, nx, ny, nz;
+};
+
+struct Binned {
+  int bx, by, bz, ghost;
+};
+
+// Bin of a cell (origin -1, edge h, floor: the reference grid) and its
+// self-ghost; folds the planarity flag, the longest cell and (when xref is
+// given) the largest squared displacement since xref into the status, one
+// atomic per warp (all lanes call; live: the lane has a cell).
+__device__ __forceinline__ Binned bin_cell(const CellsView& c, size_t i, bool live, double h, int ghost_mode,
+                                           const double* __restrict__ xref, DevStatus* st) {
+  Binned o = {0, 0, 0, 0};
+  int nonplanar = 0;
   double len = 0.0, drift2 = 0.0;
   if (live) {
     const double x = c.x[i], y = c.y[i], z = c.z[i];
-    bx = (int)floor(dvd(sub(x, -1.0), h));
-    by = (int)floor(dvd(sub(y, -1.0), h));
-    bz = (int)floor(dvd(sub(z, -1.0), h));
-    binxyz[3 * i] = bx;
-    binxyz[3 * i + 1] = by;
-    binxyz[3 * i + 2] = bz;
+    o.bx = (int)floor(dvd(sub(x, -1.0), h));
+    o.by = (int)floor(dvd(sub(y, -1.0), h));
+    o.bz = (int)floor(dvd(sub(z, -1.0), h));
     len = c.len[i];
     if (xref) {
       const double dx = x - xref[3 * i], dy = y - xref[3 * i + 1], dz = z - xref[3 * i + 2];
@@ -64,14 +87,15 @@ __global__ void k_bin(CellsView c, size_t n, double h, int ghost_mode, const dou
     }
     // planar colony (z = 0, rotation about z only): the solver may use its 2D form
     nonplanar = (z != 0.0 || c.q1[i] != 0.0 || c.q2[i] != 0.0) ? 1 : 0;
-    int g = 0;
     if (ghost_mode == PCC_GHOSTS_SINGLE_RANK) {
       // Domain::exchangeGhostParticles at world size 1 (spatial/Domain.cpp:339-403)
       // with calculateDistanceToAngularBoundary (263-290) for the sector [0, 360).
-      double ang = dvd(mul(atan2(y, x), 180.0), M_PI);
-      if (ang < 0) ang += 360.0;
-      double radius = __dsqrt_rn(add(mul(x, x), mul(y, y)));
-      if (radius >= 8.0) {
+      // The distance is |y| up to rounding (radius * sin of the angle to the x
+      // axis), so a cell well beyond 2.5 in y needs no angle.
+      const double radius = __dsqrt_rn(add(mul(x, x), mul(y, y)));
+      if (radius >= 8.0 && !(fabs(y) > 3.0 && radius < 1e9)) {
+        double ang = dvd(mul(atan2(y, x), 180.0), M_PI);
+        if (ang < 0) ang += 360.0;
         double dmin = ang - 0.0, dmax = 360.0 - ang;
         while (dmin > 180.0) dmin -= 360.0;
         while (dmin < -180.0) dmin += 360.0;
@@ -82,121 +106,147 @@ __global__ void k_bin(CellsView c, size_t n, double h, int ghost_mode, const dou
           double m = fabs(dmin) < fabs(dmax) ? fabs(dmin) : fabs(dmax);
           dist = mul(radius, sin(dvd(mul(m, M_PI), 180.0)));
         }
-        g = dist < 2.5 ? 1 : 0;
+        o.ghost = dist < 2.5 ? 1 : 0;
       }
     }
-    ghost[i] = g;
   }
-  const unsigned full = 0xffffffffu;
-  const int big = 2147483647, small = -2147483647 - 1;
-  const int mnx = __reduce_min_sync(full, live ? bx : big), mny = __reduce_min_sync(full, live ? by : big),
-            mnz = __reduce_min_sync(full, live ? bz : big);
-  const int mxx = __reduce_max_sync(full, live ? bx : small), mxy = __reduce_max_sync(full, live ? by : small),
-            mxz = __reduce_max_sync(full, live ? bz : small);
-  const unsigned np = __reduce_or_sync(full, (unsigned)nonplanar);
-  if ((threadIdx.x & 31) == 0 && mnx != big) {
-    atomicMin(&bbox[0], mnx);
-    atomicMin(&bbox[1], mny);
-    atomicMin(&bbox[2], mnz);
-    atomicMax(&bbox[3], mxx);
-    atomicMax(&bbox[4], mxy);
-    atomicMax(&bbox[5], mxz);
-    if (np) atomicOr(&bbox[6], 1);
-  }
+  const unsigned np = __reduce_or_sync(0xffffffffu, (unsigned)nonplanar);
+  if ((threadIdx.x & 31) == 0 && np) atomicOr(&st->nonplanar, 1u);
   warp_max_into(&st->lmax_bits, len);
   if (xref) warp_max_into(&st->drift_bits, drift2);
+  return o;
 }
 
-struct Grid {
-  int mx, my, mz, nx, ny, nz;
-};
-
-__device__ __forceinline__ Grid grid_from(const int* bbox) {
-  Grid g;
-  g.mx = bbox[0];
-  g.my = bbox[1];
-  g.mz = bbox[2];
-  g.nx = bbox[3] - bbox[0] + 1;
-  g.ny = bbox[4] - bbox[1] + 1;
-  g.nz = bbox[5] - bbox[2] + 1;
-  return g;
+__device__ __forceinline__ int bin_key(const Grid& g, int bx, int by, int bz) {
+  return ((bz - g.mz) * g.ny + (by - g.my)) * g.nx + (bx - g.mx);
 }
 
 // Bin counts with warp-aggregated atomics: the lanes of a warp that fall in
 // the same bin (cells are in x-sorted order, so neighbours often do) find
 // each other with __match_any_sync and one of them adds the group's size.
-__global__ void k_bin_count(const int* __restrict__ binxyz, size_t n, const int* __restrict__ bbox,
-                            int* __restrict__ key, int* __restrict__ cnt) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = i < n;
-  int k = -1;
-  if (live) {
-    const Grid g = grid_from(bbox);
-    k = ((binxyz[3 * i + 2] - g.mz) * g.ny + (binxyz[3 * i + 1] - g.my)) * g.nx + (binxyz[3 * i] - g.mx);
-    key[i] = k;
-  }
-  const unsigned peers = __match_any_sync(0xffffffffu, k);
-  const int leader = __ffs(peers) - 1;
-  if (live && (int)(threadIdx.x & 31) == leader) atomicAdd(&cnt[k], __popc(peers));
+__device__ __forceinline__ void count_bin(int k, bool live, int* __restrict__ cnt) {
+  const unsigned peers = __match_any_sync(0xffffffffu, live ? k : -1);
+  if (live && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[k], __popc(peers));
 }
 
-// Scatter into the bins: one atomic per group of same-bin lanes reserves the
-// group's slots, each lane takes the slot of its rank in the group (the order
-// inside a bin is fixed afterwards by k_segment_sort).
+// Bins every cell.  With kCount the grid is known (a box around the colony's
+// radius) and the bins are counted too; a cell outside the box raises
+// kOutOfBox and the caller starts again without it.  Otherwise the bounding
+// box of the bins is folded into the status for the caller to read.
+template <bool kCount>
+__global__ void k_bin(CellsView c, size_t n, double h, int ghost_mode, Grid g, int* __restrict__ binxyz,
+                      int* __restrict__ ghost, int* __restrict__ key, int* __restrict__ cnt, DevStatus* st) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i < n;
+  const Binned b = bin_cell(c, i, live, h, ghost_mode, nullptr, st);
+  if (live) {
+    binxyz[3 * i] = b.bx;
+    binxyz[3 * i + 1] = b.by;
+    binxyz[3 * i + 2] = b.bz;
+    ghost[i] = b.ghost;
+  }
+  if constexpr (kCount) {
+    const bool in = b.bx >= g.mx && b.bx < g.mx + g.nx && b.by >= g.my && b.by < g.my + g.ny && b.bz >= g.mz &&
+                    b.bz < g.mz + g.nz;
+    if (live && !in) atomicOr(&st->list_flags, kOutOfBox);
+    const int k = in ? bin_key(g, b.bx, b.by, b.bz) : 0;
+    if (live) key[i] = k;
+    count_bin(k, live, cnt);
+  } else {
+    const int v[3] = {b.bx, b.by, b.bz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const unsigned lo = __reduce_max_sync(0xffffffffu, live ? box_key_lo(v[d]) : 0u);
+      const unsigned hi = __reduce_max_sync(0xffffffffu, live ? box_key_hi(v[d]) : 0u);
+      if ((threadIdx.x & 31) == 0) {
+        if (lo) atomicMax(&st->box_lo[d], lo);
+        if (hi) atomicMax(&st->box_hi[d], hi);
+      }
+    }
+  }
+}
+
+__global__ void k_bin_count(const int* __restrict__ binxyz, size_t n, Grid g, int* __restrict__ key,
+                            int* __restrict__ cnt) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i < n;
+  int k = 0;
+  if (live) key[i] = k = bin_key(g, binxyz[3 * i], binxyz[3 * i + 1], binxyz[3 * i + 2]);
+  count_bin(k, live, cnt);
+}
+
+// Scatter into the bins from their ends (the counts run down to zero): one
+// atomic per group of same-bin lanes takes the group's slots, each lane the
+// slot of its rank in the group (k_pack orders each bin).
 __global__ void k_bin_scatter(const int* __restrict__ key, size_t n, const int* __restrict__ off,
-                              int* __restrict__ cursor, int* __restrict__ cells) {
+                              int* __restrict__ cnt, int* __restrict__ cells) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < n;
   const int k = live ? key[i] : -1;
   const unsigned peers = __match_any_sync(0xffffffffu, k);
   const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
   int base = 0;
-  if (live && lane == leader) base = atomicAdd(&cursor[k], __popc(peers));
+  if (live && lane == leader) base = atomicSub(&cnt[k], __popc(peers)) - __popc(peers);
   base = __shfl_sync(peers, base, leader);
   if (live) cells[off[k] + base + __popc(peers & ((1u << lane) - 1u))] = (int)i;
 }
 
-// Sort each segment [off[s], off[s+1]) ascending (segments are short).
-__global__ void k_segment_sort(const int* __restrict__ off, size_t nseg, int* __restrict__ v) {
-  size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  int b = off[s], e = off[s + 1];
-  for (int i = b + 1; i < e; ++i) {
-    int x = v[i];
-    int j = i - 1;
-    while (j >= b && v[j] > x) {
-      v[j + 1] = v[j];
-      --j;
-    }
-    v[j + 1] = x;
-  }
-}
-
-__global__ void k_pack(CellsView c, const int* __restrict__ slot_cell, const int* __restrict__ ghost, size_t n,
-                       double* __restrict__ pk) {
-  size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  int i = slot_cell[s];
+// Packs cell i's record at slot s.
+__device__ __forceinline__ void pack_cell(const CellsView& c, int i, int ghost, size_t s, double* __restrict__ pk) {
   double t[3];
   cell_axis(c.q0[i], c.q1[i], c.q2[i], c.q3[i], t);
   const double len = c.len[i], diam = c.diam[i];
   // CollisionDetector::getParticleEndpoints (spatial/CollisionDetector.cpp:61-75)
   const double half = sub(dvd(len, 2.0), dvd(diam, 2.0));
   const double p[3] = {c.x[i], c.y[i], c.z[i]};
-  double* r = pk + s * kPack;
+  double r[kPack];
   r[0] = p[0];
   r[1] = p[1];
   r[2] = p[2];
   r[3] = len;
   for (int d = 0; d < 3; ++d) {
-    double hv = mul(t[d], half);
+    const double hv = mul(t[d], half);
     r[4 + d] = sub(p[d], hv);
     r[8 + d] = add(p[d], hv);
     r[12 + d] = t[d];
   }
   r[7] = diam;
   r[11] = (double)i;
-  r[15] = (double)ghost[i];
+  r[15] = (double)ghost;
+  double2* o = reinterpret_cast<double2*>(pk + s * kPack);
+#pragma unroll
+  for (int q = 0; q < kPack / 2; ++q) o[q] = make_double2(r[2 * q], r[2 * q + 1]);
+}
+
+// Orders each bin by id and packs the records in that order: thread per
+// scattered cell, whose rank among its bin's cells is its slot there.
+__global__ void k_pack(CellsView c, const int* __restrict__ raw, const int* __restrict__ key,
+                       const int* __restrict__ off, const int* __restrict__ ghost, size_t n, int* __restrict__ slot_cell,
+                       int* __restrict__ slot_of, double* __restrict__ pk) {
+  const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int i = raw[r], k = key[i], e = off[k + 1];
+  int s = off[k];
+  for (int q = s; q < e; ++q) s += raw[q] < i ? 1 : 0;
+  slot_cell[s] = i;
+  slot_of[i] = s;
+  pack_cell(c, i, ghost[i], (size_t)s, pk);
+}
+
+// Later ReLCP phase on the slots of the pass that built the lists: current
+// bins, ghosts and records in one pass.
+__global__ void k_repack(CellsView c, const int* __restrict__ slot_cell, size_t n, double h, int ghost_mode,
+                         const double* __restrict__ xref, int* __restrict__ binxyz, double* __restrict__ pk,
+                         DevStatus* st) {
+  const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = s < n;
+  const size_t i = live ? (size_t)slot_cell[s] : 0;
+  const Binned b = bin_cell(c, i, live, h, ghost_mode, xref, st);
+  if (!live) return;
+  binxyz[3 * i] = b.bx;
+  binxyz[3 * i + 1] = b.by;
+  binxyz[3 * i + 2] = b.bz;
+  pack_cell(c, (int)i, b.ghost, s, pk);
 }
 
 // Closest points of two segments: Eberly's branch scheme for segment-segment
@@ -410,87 +460,109 @@ __device__ __forceinline__ bool emit_rows(ConsView cs, size_t& w, size_t cap, in
   return true;
 }
 
-// Bin of the cell at slot s: the last bin whose offset is <= s.
-__device__ __forceinline__ int bin_of_slot(const int* __restrict__ bin_off, int nbins, int s) {
-  int lo = 0, hi = nbins;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (bin_off[mid] <= s) lo = mid;
-    else hi = mid;
-  }
-  return lo;
+// Slots [lo, hi) of the up to three bins of stencil row (dy, dz) of a cell at
+// bin (bx, by, bz) (grid coordinates): they hold consecutive slots.
+__device__ __forceinline__ bool stencil_row(const Grid& g, const int* __restrict__ bin_off, int bx, int y, int z,
+                                            int* lo, int* hi) {
+  if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) return false;
+  const int x0 = bx > 0 ? bx - 1 : 0, x1 = bx + 1 < g.nx ? bx + 1 : g.nx - 1;
+  const int row = (z * g.ny + y) * g.nx;
+  *lo = bin_off[row + x0];
+  *hi = bin_off[row + x1 + 1];
+  return true;
 }
 
-// Full neighbourhood pass of a phase: one thread per cell in bin order scans
-// the 27-stencil for partners with a larger id (the candidate pairs of
-// SpatialGrid::findPotentialCollisions, spatial/SpatialGrid.cpp:58-121).  For
-// each pair that passes tryCreateConstraint it counts the constraints the
-// smaller id emits (a second copy when the partner has a self-ghost), tracks
-// the largest overlap, and adds to Particle::num_constraints of both cells
-// (CollisionDetector.cpp:243-244, ghost copies included; the count of a cell
-// that has a self-ghost lands on the copy and is lost, as in the reference).
-// Every partner within the wider reach tol_list is appended to the cell's
-// candidate list (slots of the packed records, stored list-major), so the
-// emit pass and the later ReLCP phases of the step need no stencil scan.
-// The cell's position at list time is kept in xref.
-__global__ void k_scan_count(const double* __restrict__ pk, const int* __restrict__ bin_off,
-                             const int* __restrict__ bbox, size_t n, double tol, double tol_list,
-                             int* __restrict__ cnt, int* __restrict__ ncontacts, int* __restrict__ plist,
-                             int* __restrict__ plist_n, double* __restrict__ xref, DevStatus* st) {
-  const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Full neighbourhood pass of a phase: kPairLanes lanes per cell in bin order
+// scan the 27-stencil for partners with a larger id (the candidate pairs of
+// SpatialGrid::findPotentialCollisions, spatial/SpatialGrid.cpp:58-121) and
+// append every partner within the wider reach tol_list to the cell's candidate
+// list (slots of the packed records) in stencil order, so the emit pass and
+// the later ReLCP phases of the step need no stencil scan.  The lanes then
+// share the listed pairs, so that the geometry runs with all lanes in use:
+// for each pair that passes tryCreateConstraint they count the constraints
+// the smaller id emits (a second copy when the partner has a self-ghost),
+// track the largest overlap, and add to Particle::num_constraints of both
+// cells (CollisionDetector.cpp:243-244, ghost copies included; the count of a
+// cell that has a self-ghost lands on the copy and is lost, as in the
+// reference).  The cell's position at list time is kept in xref.
+template <int kPairLanes>
+__global__ void __launch_bounds__(kBlock) k_scan_count(const double* __restrict__ pk, const int* __restrict__ bin_off,
+                                                       Grid g, const int* __restrict__ binxyz, size_t n, double tol,
+                                                       double tol_list, int* __restrict__ cnt,
+                                                       int* __restrict__ ncontacts, int* __restrict__ plist,
+                                                       int* __restrict__ plist_n, double* __restrict__ xref,
+                                                       DevStatus* st) {
+  static_assert(kPairLanes >= 3, "three lanes write the position");
+  __shared__ int s_list[kBlock / kPairLanes][kList];
+  const size_t s = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kPairLanes;
+  const int lane = threadIdx.x & 31, l = lane % kPairLanes, shift = lane - l;
+  constexpr unsigned kOnes = kPairLanes == 32 ? ~0u : (1u << kPairLanes) - 1u;
+  const unsigned group = kOnes << shift;
+  int* list = s_list[threadIdx.x / kPairLanes];
+  if (__ldcg(&st->list_flags) & kOutOfBox) return;  // the binning failed: count nothing
   double maxov = 0.0;
   if (s < n) {
-    const Grid g = grid_from(bbox);
     const double* A = pk + s * kPack;
     const int a = (int)A[11];
     const double4 a0 = *reinterpret_cast<const double4*>(A);
-    xref[3 * (size_t)a] = a0.x;
-    xref[3 * (size_t)a + 1] = a0.y;
-    xref[3 * (size_t)a + 2] = a0.z;
-    const int bin = bin_of_slot(bin_off, g.nx * g.ny * g.nz, (int)s);
-    const int bx = bin % g.nx, by = (bin / g.nx) % g.ny, bz = bin / (g.nx * g.ny);
+    if (l < 3) xref[3 * (size_t)a + l] = A[l];
+    const int bx = binxyz[3 * (size_t)a] - g.mx, by = binxyz[3 * (size_t)a + 1] - g.my,
+              bz = binxyz[3 * (size_t)a + 2] - g.mz;
     const int ga = A[15] != 0.0;
     int count = 0, nl = 0;
+    auto test = [&](const double* B, int b) {
+      PairGeom pg;
+      if (!pair_geom(A, B, tol, false, &pg)) return;
+      const int gb = B[15] != 0.0;
+      count += 1 + gb;
+      const double ov = pg.sd < 0 ? -pg.sd : 0.0;
+      maxov = maxov < ov ? ov : maxov;
+      if (!gb) atomicAdd(&ncontacts[b], 1 + ga);
+    };
     for (int dz = -1; dz <= 1; ++dz) {
-      const int z = bz + dz;
-      if (z < 0 || z >= g.nz) continue;
       for (int dy = -1; dy <= 1; ++dy) {
-        const int y = by + dy;
-        if (y < 0 || y >= g.ny) continue;
-        // the (up to) three bins of a stencil row hold consecutive slots
-        const int x0 = bx > 0 ? bx - 1 : 0, x1 = bx + 1 < g.nx ? bx + 1 : g.nx - 1;
-        const int row = (z * g.ny + y) * g.nx;
-        const int e = bin_off[row + x1 + 1];
-        for (int s2 = bin_off[row + x0]; s2 < e; ++s2) {
+        int lo, hi;
+        if (!stencil_row(g, bin_off, bx, by + dy, bz + dz, &lo, &hi)) continue;
+        for (int s0 = lo; s0 < hi; s0 += kPairLanes) {
+          const int s2 = s0 + l;
           const double* B = pk + (size_t)s2 * kPack;
-          const int b = (int)B[11];
-          if (b <= a) continue;
-          const double4 b0 = *reinterpret_cast<const double4*>(B);
-          if (!rough_pass(a0, b0, tol_list)) continue;
-          if (nl < kList) plist[(size_t)nl * n + a] = s2;
-          ++nl;
-          if (tol < tol_list && !rough_pass(a0, b0, tol)) continue;
-          PairGeom pg;
-          if (!pair_geom(A, B, tol, false, &pg)) continue;
-          const int gb = B[15] != 0.0;
-          count += 1 + gb;
-          const double ov = pg.sd < 0 ? -pg.sd : 0.0;
-          maxov = maxov < ov ? ov : maxov;
-          if (!ga) atomicAdd(&ncontacts[a], 1 + gb);
-          if (!gb) atomicAdd(&ncontacts[b], 1 + ga);
+          bool in = false;
+          if (s2 < hi && (int)B[11] > a) in = rough_pass(a0, *reinterpret_cast<const double4*>(B), tol_list);
+          const unsigned hits = __ballot_sync(group, in) >> shift & kOnes;
+          const int at = nl + __popc(hits & ((1u << l) - 1u));
+          nl += __popc(hits);
+          if (!in) continue;
+          if (at < kList) {
+            list[at] = s2;
+            plist[(size_t)a * kList + at] = s2;
+          } else if (!(tol < tol_list) || rough_pass(a0, *reinterpret_cast<const double4*>(B), tol)) {
+            test(B, (int)B[11]);  // no room in the list
+          }
         }
       }
     }
-    cnt[a] = count;
-    plist_n[a] = nl;
-    if (nl > kList) atomicOr(&st->list_flags, kListOverflow);
+    __syncwarp(group);
+    const int listed = nl < kList ? nl : kList;
+    for (int k = l; k < listed; k += kPairLanes) {
+      const double* B = pk + (size_t)list[k] * kPack;
+      if (tol < tol_list && !rough_pass(a0, *reinterpret_cast<const double4*>(B), tol)) continue;
+      test(B, (int)B[11]);
+    }
+#pragma unroll
+    for (int o = kPairLanes / 2; o > 0; o >>= 1) count += __shfl_xor_sync(group, count, o);
+    if (l == 0) {
+      cnt[a] = count;
+      if (!ga && count) atomicAdd(&ncontacts[a], count);
+      plist_n[a] = nl;
+      if (nl > kList) atomicOr(&st->list_flags, kListOverflow);
+    }
   }
   warp_max_into(&st->max_bits, maxov);
 }
 
-// Count (kEmit = false) or emit pass over the candidate lists, one thread per
-// cell in id order; the emit order per cell is the list order, which is the
-// stencil order of the full pass.
+// Count (kEmit = false) or emit pass over the candidate lists, kPairLanes
+// lanes per cell in id order; the emit order per cell is the list order,
+// which is the stencil order of the full pass.
 //
 // In a later ReLCP phase of the step (adjacent = true) the lists are reused
 // without rebinning the colony.  A listed pair is a candidate only if the two
@@ -502,22 +574,25 @@ __global__ void k_scan_count(const double* __restrict__ pk, const int* __restric
 // than one bin edge h (so in neighbouring bins) when L + tol + 2D < h.  If
 // either bound fails the pass does nothing and flags the lists stale; the
 // caller then runs the full pass.
-template <bool kEmit>
-__global__ void k_list_pass(const double* __restrict__ pk, const int* __restrict__ slot_of, size_t n, double tol,
-                            int phase, bool adjacent, double tol_list, double h, const int* __restrict__ binxyz,
-                            const int* __restrict__ plist, const int* __restrict__ plist_n, int* __restrict__ cnt,
-                            int* __restrict__ ncontacts, const int* __restrict__ off, ConsView cs, size_t base,
-                            size_t cap, DevStatus* st) {
-  const size_t a = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+template <bool kEmit, int kPairLanes>
+__global__ void __launch_bounds__(kBlock) k_list_pass(
+    const double* __restrict__ pk, const int* __restrict__ slot_of, size_t n, double tol, int phase, bool adjacent,
+    double tol_list, double h, const int* __restrict__ binxyz, const int* __restrict__ plist,
+    const int* __restrict__ plist_n, int* __restrict__ cnt, int* __restrict__ ncontacts, const int* __restrict__ off,
+    ConsView cs, size_t base, size_t cap, DevStatus* st) {
+  const size_t a = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kPairLanes;
   if (!kEmit && adjacent) {
     const double d2 = __longlong_as_double((long long)__ldcg(&st->drift_bits));
     const double lmax = __longlong_as_double((long long)__ldcg(&st->lmax_bits));
     const double reach = tol + 2.0 * sqrt(d2);
     if (!(reach < tol_list - 1e-6 && lmax + reach < h - 1e-6)) {
-      if (a == 0) atomicOr(&st->list_flags, kListStale);
+      if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&st->list_flags, kListStale);
       return;
     }
   }
+  const int lane = threadIdx.x & 31, l = lane % kPairLanes, shift = lane - l;
+  constexpr unsigned kOnes = kPairLanes == 32 ? ~0u : (1u << kPairLanes) - 1u;
+  const unsigned group = kOnes << shift;
   double maxov = 0.0;
   if (a < n) {
     const double* A = pk + (size_t)slot_of[a] * kPack;
@@ -532,58 +607,66 @@ __global__ void k_list_pass(const double* __restrict__ pk, const int* __restrict
     }
     int count = 0;
     size_t w = kEmit ? base + (size_t)off[a] : 0;
-    for (int k = 0; k < nl; ++k) {
-      const int s2 = plist[(size_t)k * n + a];
-      const double* B = pk + (size_t)s2 * kPack;
-      const int b = (int)B[11];
-      if (adjacent) {
-        const int ex = binxyz[3 * (size_t)b] - bxa, ey = binxyz[3 * (size_t)b + 1] - bya,
-                  ez = binxyz[3 * (size_t)b + 2] - bza;
-        if (ex < -1 || ex > 1 || ey < -1 || ey > 1 || ez < -1 || ez > 1) continue;
-      }
-      const double4 b0 = *reinterpret_cast<const double4*>(B);
-      if (!rough_pass(a0, b0, tol)) continue;
+    for (int k0 = 0; k0 < nl; k0 += kPairLanes) {
+      const int k = k0 + l;
+      int b = 0, gb = 0;
+      bool pass = false;
       PairGeom pg;
-      if (!pair_geom(A, B, tol, kEmit, &pg)) continue;
-      const int gb = B[15] != 0.0;
+      if (k < nl) {
+        const double* B = pk + (size_t)plist[a * kList + k] * kPack;
+        b = (int)B[11];
+        pass = true;
+        if (adjacent) {
+          const int ex = binxyz[3 * (size_t)b] - bxa, ey = binxyz[3 * (size_t)b + 1] - bya,
+                    ez = binxyz[3 * (size_t)b + 2] - bza;
+          pass = ex >= -1 && ex <= 1 && ey >= -1 && ey <= 1 && ez >= -1 && ez <= 1;
+        }
+        pass = pass && rough_pass(a0, *reinterpret_cast<const double4*>(B), tol);
+        pass = pass && pair_geom(A, B, tol, kEmit, &pg);
+        gb = pass && B[15] != 0.0;
+      }
       if (kEmit) {
-        if (!emit_rows(cs, w, cap, (int)a, b, phase, 1 + gb, pg, st)) break;
-      } else {
+        const unsigned low = (1u << l) - 1u;
+        const unsigned p = __ballot_sync(group, pass) >> shift, g2 = __ballot_sync(group, gb) >> shift;
+        size_t at = w + __popc(p & low) + __popc(g2 & low);
+        if (pass) emit_rows(cs, at, cap, (int)a, b, phase, 1 + gb, pg, st);
+        w += __popc(p & kOnes) + __popc(g2 & kOnes);
+      } else if (pass) {
         count += 1 + gb;
         const double ov = pg.sd < 0 ? -pg.sd : 0.0;
         maxov = maxov < ov ? ov : maxov;
-        if (!ga) atomicAdd(&ncontacts[a], 1 + gb);
         if (!gb) atomicAdd(&ncontacts[b], 1 + ga);
       }
     }
-    if (!kEmit) cnt[a] = count;
+    if (!kEmit) {
+#pragma unroll
+      for (int o = kPairLanes / 2; o > 0; o >>= 1) count += __shfl_xor_sync(group, count, o);
+      if (l == 0) {
+        cnt[a] = count;
+        if (!ga && count) atomicAdd(&ncontacts[a], count);
+      }
+    }
   }
   if (!kEmit) warp_max_into(&st->max_bits, maxov);
 }
 
 // Emit pass over the 27-stencil, for a phase whose candidate lists overflowed.
-__global__ void k_stencil_emit(const double* __restrict__ pk, const int* __restrict__ bin_off,
-                               const int* __restrict__ bbox, size_t n, double tol, int phase,
+__global__ void k_stencil_emit(const double* __restrict__ pk, const int* __restrict__ bin_off, Grid g,
+                               const int* __restrict__ binxyz, size_t n, double tol, int phase,
                                const int* __restrict__ off, ConsView cs, size_t base, size_t cap, DevStatus* st) {
   const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  const Grid g = grid_from(bbox);
   const double* A = pk + s * kPack;
   const int a = (int)A[11];
   const double4 a0 = *reinterpret_cast<const double4*>(A);
-  const int bin = bin_of_slot(bin_off, g.nx * g.ny * g.nz, (int)s);
-  const int bx = bin % g.nx, by = (bin / g.nx) % g.ny, bz = bin / (g.nx * g.ny);
+  const int bx = binxyz[3 * (size_t)a] - g.mx, by = binxyz[3 * (size_t)a + 1] - g.my,
+            bz = binxyz[3 * (size_t)a + 2] - g.mz;
   size_t w = base + (size_t)off[a];
   for (int dz = -1; dz <= 1; ++dz) {
-    const int z = bz + dz;
-    if (z < 0 || z >= g.nz) continue;
     for (int dy = -1; dy <= 1; ++dy) {
-      const int y = by + dy;
-      if (y < 0 || y >= g.ny) continue;
-      const int x0 = bx > 0 ? bx - 1 : 0, x1 = bx + 1 < g.nx ? bx + 1 : g.nx - 1;
-      const int row = (z * g.ny + y) * g.nx;
-      const int e = bin_off[row + x1 + 1];
-      for (int s2 = bin_off[row + x0]; s2 < e; ++s2) {
+      int lo, hi;
+      if (!stencil_row(g, bin_off, bx, by + dy, bz + dz, &lo, &hi)) continue;
+      for (int s2 = lo; s2 < hi; ++s2) {
         const double* B = pk + (size_t)s2 * kPack;
         const int b = (int)B[11];
         if (b <= a) continue;
@@ -597,9 +680,20 @@ __global__ void k_stencil_emit(const double* __restrict__ pk, const int* __restr
   }
 }
 
-__global__ void k_slot_of(const int* __restrict__ slot_cell, size_t n, int* __restrict__ slot_of) {
-  const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n) slot_of[slot_cell[s]] = (int)s;
+// Sort each segment [off[s], off[s+1]) ascending (segments are short).
+__global__ void k_segment_sort(const int* __restrict__ off, size_t nseg, int* __restrict__ v) {
+  size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nseg) return;
+  int b = off[s], e = off[s + 1];
+  for (int i = b + 1; i < e; ++i) {
+    int x = v[i];
+    int j = i - 1;
+    while (j >= b && v[j] > x) {
+      v[j + 1] = v[j];
+      --j;
+    }
+    v[j + 1] = x;
+  }
 }
 
 __global__ void k_inc_count(const int* __restrict__ gi, const int* __restrict__ gj, size_t m, int* __restrict__ cnt) {
@@ -620,6 +714,21 @@ __global__ void k_inc_fill(const int* __restrict__ gi, const int* __restrict__ g
 
 }  // namespace
 
+// Grid of the bins of every centre within `r` of the origin, if it is not too
+// large for the colony (a long chain's box would be mostly empty); at z the
+// one bin of the plane z = 0.
+static bool box_of_radius(double r, double h, size_t n, Grid* g) {
+  if (!(r >= 0) || !(r < 1e8 * h)) return false;
+  const int lo = (int)std::floor((-r + 1.0) / h) - 1, hi = (int)std::floor((r + 1.0) / h) + 1;
+  const long long w = (long long)hi - lo + 1;
+  if (w * w > 8 * (long long)n + 16384) return false;
+  g->mx = g->my = lo;
+  g->nx = g->ny = (int)w;
+  g->mz = (int)std::floor(1.0 / h);
+  g->nz = 1;
+  return true;
+}
+
 cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, size_t* added,
                             double* max_overlap_new) {
   cudaStream_t s = ctx->stream;
@@ -629,15 +738,21 @@ cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, siz
   *max_overlap_new = 0.0;
   if (!reuse) ctx->list_valid = false;
   if (n == 0) return cudaSuccess;
-  int* pinned = reinterpret_cast<int*>(ctx->pinned_ll);
-  static const int init[7] = {2147483647, 2147483647, 2147483647, -2147483647 - 1, -2147483647 - 1,
-                              -2147483647 - 1, 0};
   const double h = ctx->params.linked_cell_size;
   const double tol_list = tol > kListReach ? tol : kListReach;
+  const int ghosts = ctx->params.ghost_mode;
+  const int lanes = n < (size_t)kFewCells ? 8 : 4;
+  const unsigned pair_grid = grid_for((long long)n * lanes);
   bool use_list = reuse && ctx->list_valid && ctx->list_n == n;
+  // the radius of the last step (or upload) bounds the centres at the start
+  // of a step -- it is the largest distance of a cell's leading end, so a
+  // centre is at most half a cell further out and a new daughter's a quarter
+  // more -- which saves the round trip for the bins' bounding box; a colony
+  // that left the plane z = 0 once does not try again
+  Grid g{};
+  bool boxed = !reuse && ctx->box_known && ctx->flat && box_of_radius(ctx->radius + 2 * ctx->params.l0, h, n, &g);
   if ((e = ctx->bin_of.reserve(3 * n, 0, s))) return e;
   if ((e = ctx->ghost.reserve(n, 0, s))) return e;
-  if ((e = ctx->bbox.reserve(8, 0, s))) return e;
   if ((e = ctx->cand_cnt.reserve(n + 1, 0, s))) return e;
   if ((e = ctx->cand_off.reserve(n + 1, 0, s))) return e;
   if ((e = ctx->pk.reserve(n * kPack, 0, s))) return e;
@@ -645,62 +760,70 @@ cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, siz
   if ((e = ctx->plist_n.reserve(n + 1, 0, s))) return e;
   if ((e = ctx->slot_of.reserve(n + 1, 0, s))) return e;
   if ((e = ctx->xref.reserve(3 * n, 0, s))) return e;
+  if ((e = ctx->bin_cells.reserve(n, 0, s))) return e;
+  if ((e = ctx->bin_raw.reserve(n, 0, s))) return e;
   for (;;) {
-    cudaMemcpyAsync(ctx->bbox.p, init, sizeof init, cudaMemcpyHostToDevice, s);  // pageable: staged at once
-    cudaMemsetAsync(&ctx->status->max_bits, 0, sizeof(unsigned long long), s);
-    cudaMemsetAsync(&ctx->status->list_flags, 0, 3 * sizeof(unsigned long long), s);
-    k_bin<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), n, h, ctx->params.ghost_mode,
-                                          use_list ? ctx->xref.p : nullptr, ctx->bin_of.p, ctx->bbox.p, ctx->ghost.p,
-                                          ctx->status);
-    ctx->launches++;
+    cudaMemsetAsync(reinterpret_cast<char*>(ctx->status) + kDetectBegin, 0, kDetectBytes, s);
     if (use_list) {
       // the slots of the pass that built the lists: bin_cells still maps slot -> cell
-      k_pack<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->bin_cells.p, ctx->ghost.p, n, ctx->pk.p);
-      k_list_pass<false><<<grid_for(n), kBlock, 0, s>>>(
+      k_repack<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->bin_cells.p, n, h, ghosts, ctx->xref.p,
+                                              ctx->bin_of.p, ctx->pk.p, ctx->status);
+      (lanes == 8 ? k_list_pass<false, 8> : k_list_pass<false, 4>)<<<pair_grid, kBlock, 0, s>>>(
           ctx->pk.p, ctx->slot_of.p, n, tol, phase, true, ctx->list_tol, h, ctx->bin_of.p, ctx->plist.p,
           ctx->plist_n.p, ctx->cand_cnt.p, ctx->cells.ncons.p, nullptr, ConsView{}, 0, 0, ctx->status);
       ctx->launches += 2;
     } else {
-      cudaMemcpyAsync(pinned, ctx->bbox.p, 7 * sizeof(int), cudaMemcpyDeviceToHost, s);
-      if ((e = cudaStreamSynchronize(s))) return e;
-      ctx->planar = pinned[6] == 0;
-      const long long nx = (long long)pinned[3] - pinned[0] + 1, ny = (long long)pinned[4] - pinned[1] + 1,
-                      nz = (long long)pinned[5] - pinned[2] + 1;
-      const long long nbins = nx * ny * nz;
-      if (nbins <= 0 || nbins > (1LL << 30)) {
-        ctx->err = "broadphase grid too large (cells spread over more than 2^30 bins)";
-        return cudaErrorInvalidValue;
-      }
-      if ((e = ctx->bin_cnt.reserve(nbins + 1, 0, s))) return e;
-      if ((e = ctx->bin_cursor.reserve(nbins + 1, 0, s))) return e;
-      if ((e = ctx->bin_off.reserve(nbins + 1, 0, s))) return e;
-      if ((e = ctx->bin_cells.reserve(n, 0, s))) return e;
       int* key = ctx->cand_cnt.p;  // per-cell bin key until the pair pass
-      cudaMemsetAsync(ctx->bin_cnt.p, 0, (nbins + 1) * sizeof(int), s);
-      cudaMemsetAsync(ctx->bin_cursor.p, 0, (nbins + 1) * sizeof(int), s);
-      k_bin_count<<<grid_for(n), kBlock, 0, s>>>(ctx->bin_of.p, n, ctx->bbox.p, key, ctx->bin_cnt.p);
-      if ((e = exclusive_scan(ctx, ctx->bin_cnt.p, ctx->bin_off.p, (size_t)nbins))) return e;
-      k_bin_scatter<<<grid_for(n), kBlock, 0, s>>>(key, n, ctx->bin_off.p, ctx->bin_cursor.p, ctx->bin_cells.p);
-      k_segment_sort<<<grid_for(nbins), kBlock, 0, s>>>(ctx->bin_off.p, (size_t)nbins, ctx->bin_cells.p);
-      k_pack<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->bin_cells.p, ctx->ghost.p, n, ctx->pk.p);
-      k_slot_of<<<grid_for(n), kBlock, 0, s>>>(ctx->bin_cells.p, n, ctx->slot_of.p);
-      k_scan_count<<<grid_for(n), kBlock, 0, s>>>(ctx->pk.p, ctx->bin_off.p, ctx->bbox.p, n, tol, tol_list,
-                                                   ctx->cand_cnt.p, ctx->cells.ncons.p, ctx->plist.p,
-                                                   ctx->plist_n.p, ctx->xref.p, ctx->status);
-      ctx->launches += 6;
+      if (!boxed) {
+        k_bin<false><<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), n, h, ghosts, g, ctx->bin_of.p, ctx->ghost.p,
+                                                    nullptr, nullptr, ctx->status);
+        ctx->launches++;
+        cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
+        if ((e = cudaStreamSynchronize(s))) return e;
+        const DevStatus& st = *ctx->status_host;
+        auto lo = [&](int d) { return (long long)(int)(~st.box_lo[d] ^ 0x80000000u); };
+        auto hi = [&](int d) { return (long long)(int)(st.box_hi[d] ^ 0x80000000u); };
+        const long long nx = hi(0) - lo(0) + 1, ny = hi(1) - lo(1) + 1, nz = hi(2) - lo(2) + 1;
+        const long long most = 1LL << 30;
+        if (nx <= 0 || ny <= 0 || nz <= 0 || nx > most || ny > most || nz > most || nx * ny > most ||
+            nx * ny * nz > most) {
+          ctx->err = "broadphase grid too large (cells spread over more than 2^30 bins)";
+          return cudaErrorInvalidValue;
+        }
+        g = Grid{(int)lo(0), (int)lo(1), (int)lo(2), (int)nx, (int)ny, (int)nz};
+      }
+      const size_t nbins = (size_t)g.nx * g.ny * g.nz;
+      if ((e = ctx->bin_cnt.reserve(nbins + 1, 0, s))) return e;
+      if ((e = ctx->bin_off.reserve(nbins + 1, 0, s))) return e;
+      cudaMemsetAsync(ctx->bin_cnt.p, 0, nbins * sizeof(int), s);
+      if (boxed)
+        k_bin<true><<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), n, h, ghosts, g, ctx->bin_of.p, ctx->ghost.p,
+                                                   key, ctx->bin_cnt.p, ctx->status);
+      else
+        k_bin_count<<<grid_for(n), kBlock, 0, s>>>(ctx->bin_of.p, n, g, key, ctx->bin_cnt.p);
+      if ((e = exclusive_scan(ctx, ctx->bin_cnt.p, ctx->bin_off.p, nbins))) return e;
+      k_bin_scatter<<<grid_for(n), kBlock, 0, s>>>(key, n, ctx->bin_off.p, ctx->bin_cnt.p, ctx->bin_raw.p);
+      k_pack<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->bin_raw.p, key, ctx->bin_off.p, ctx->ghost.p, n,
+                                            ctx->bin_cells.p, ctx->slot_of.p, ctx->pk.p);
+      (lanes == 8 ? k_scan_count<8> : k_scan_count<4>)<<<pair_grid, kBlock, 0, s>>>(ctx->pk.p, ctx->bin_off.p, g, ctx->bin_of.p, n, tol, tol_list,
+                                                ctx->cand_cnt.p, ctx->cells.ncons.p, ctx->plist.p, ctx->plist_n.p,
+                                                ctx->xref.p, ctx->status);
+      ctx->launches += 4;
     }
-    if ((e = exclusive_scan(ctx, ctx->cand_cnt.p, ctx->cand_off.p, n))) return e;
-    cudaMemcpyAsync(pinned, ctx->cand_off.p + n, sizeof(int), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->pinned_ll + 1, &ctx->status->max_bits, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                    s);
-    cudaMemcpyAsync(pinned + 4, &ctx->status->list_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    // k_bin folds the planarity of the current cells on every pass: cells
-    // that left the plane since the last full pass (out-of-plane Brownian
-    // kicks) must take the general solver
-    cudaMemcpyAsync(pinned + 5, ctx->bbox.p + 6, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if ((e = exclusive_scan(ctx, ctx->cand_cnt.p, ctx->cand_off.p, n, &ctx->status->count))) return e;
+    cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s))) return e;
-    ctx->planar = pinned[5] == 0;
-    const unsigned flags = (unsigned)pinned[4];
+    const DevStatus& st = *ctx->status_host;
+    const unsigned flags = st.list_flags;
+    if (!use_list && boxed && (flags & kOutOfBox)) {
+      // a cell outside the assumed box: nothing was counted, start again
+      boxed = false;
+      if (st.nonplanar) ctx->flat = false;
+      continue;
+    }
+    // cells that left the plane since the last full pass (out-of-plane
+    // Brownian kicks) must take the general solver
+    ctx->planar = st.nonplanar == 0;
     if (use_list && (flags & kListStale)) {
       // cells moved too far since the lists were built: rebin this phase
       use_list = false;
@@ -715,21 +838,18 @@ cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, siz
       ctx->list_n = n;
       ctx->list_tol = tol_list;
     }
-    const size_t m = (size_t)pinned[0];
-    unsigned long long bits = (unsigned long long)ctx->pinned_ll[1];
-    double mo;
-    memcpy(&mo, &bits, sizeof mo);
-    *max_overlap_new = mo;
+    const size_t m = (size_t)st.count;
+    memcpy(max_overlap_new, &st.max_bits, sizeof *max_overlap_new);
     *added = m;
     if (m == 0) return cudaSuccess;
     if ((e = ctx->cons.reserve(ctx->ncons + m, ctx->ncons, s))) return e;
     if (listed) {
-      k_list_pass<true><<<grid_for(n), kBlock, 0, s>>>(ctx->pk.p, ctx->slot_of.p, n, tol, phase, use_list, tol_list,
-                                                      h, ctx->bin_of.p, ctx->plist.p, ctx->plist_n.p, nullptr,
-                                                      nullptr, ctx->cand_off.p, ctx->cons.view(), ctx->ncons,
-                                                      ctx->ncons + m, ctx->status);
+      (lanes == 8 ? k_list_pass<true, 8> : k_list_pass<true, 4>)<<<pair_grid, kBlock, 0, s>>>(ctx->pk.p, ctx->slot_of.p, n, tol, phase, use_list, tol_list, h,
+                                                    ctx->bin_of.p, ctx->plist.p, ctx->plist_n.p, nullptr, nullptr,
+                                                    ctx->cand_off.p, ctx->cons.view(), ctx->ncons, ctx->ncons + m,
+                                                    ctx->status);
     } else {
-      k_stencil_emit<<<grid_for(n), kBlock, 0, s>>>(ctx->pk.p, ctx->bin_off.p, ctx->bbox.p, n, tol, phase,
+      k_stencil_emit<<<grid_for(n), kBlock, 0, s>>>(ctx->pk.p, ctx->bin_off.p, g, ctx->bin_of.p, n, tol, phase,
                                                     ctx->cand_off.p, ctx->cons.view(), ctx->ncons, ctx->ncons + m,
                                                     ctx->status);
     }

@@ -7,11 +7,9 @@
 
 namespace pcc {
 
-// Slots of ctx->pinned_ll for values copied back at a synchronisation point
-// (slots 0..7 belong to the detection pass).
+// Slots of ctx->pinned_ll for values copied back at a synchronisation point.
 constexpr int kSlotRadius = 10;  // colony radius bits
 constexpr int kSlotDivs = 11;    // divisions of the next step
-constexpr int kSlotMaxOld = 12;  // largest overlap of the earlier phases' constraints
 
 // ---- pcc_scan_sort.cu
 // out[i] = sum in[0..i-1] for i in [0, n]; out has n+1 entries.  The sum of
@@ -38,13 +36,11 @@ cudaError_t build_incidence(pcc_ctx* ctx);
 cudaError_t brownian_draw(pcc_ctx* ctx);
 // One BBPGD solve on the current constraint set (hard model).  With defer,
 // only launches it and enqueues the copy of its scalars (ctx->bbpgd_pending);
-// bbpgd_collect reads them after the caller's next synchronisation.
+// bbpgd_collect reads them after the caller's next synchronisation that also
+// copied the device status.  It sets ctx->solved_overlap.
 cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* residual, int* status,
                         bool defer = false);
 void bbpgd_collect(pcc_ctx* ctx, long long* iterations, double* residual, int* status);
-// Largest overlap of constraints [from, to) into ctx->pinned_ll[kSlotMaxOld]
-// at the next synchronisation (no host wait).
-cudaError_t max_overlap_enqueue(pcc_ctx* ctx, size_t from, size_t to);
 // Moves cells with the solver's velocities and writes back gamma / phi.
 cudaError_t apply_hard_solution(pcc_ctx* ctx, double dt);
 // Soft model: Hertz forces, motion and growth parameters.

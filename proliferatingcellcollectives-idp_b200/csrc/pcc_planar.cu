@@ -461,7 +461,13 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
     if (recorder) sc->iterations = it;
     if (!conv) return;
     const long long tid = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)nb * kBlock;
-    for (long long c = tid; c < a.m; c += stride) a.phi[c] = ldcg(a.phin + c);
+    double most = 0.0;
+    for (long long c = tid; c < a.m; c += stride) {
+      const double phi = ldcg(a.phin + c);
+      a.phi[c] = phi;
+      most = overlap_of(most, phi);
+    }
+    fold_overlap(sc, most);
     return;
   }
 
@@ -527,7 +533,13 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
   // returned result (Hard.cpp:170 with BBPGD.cpp:124): gamma_{k-1} (stored by
   // the last constraint pass), phi of gamma_k
   const long long tid = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)nb * kBlock;
-  for (long long c = tid; c < a.m; c += stride) a.phi[c] = ldcg(a.phin + c);
+  double most = 0.0;
+  for (long long c = tid; c < a.m; c += stride) {
+    const double phi = ldcg(a.phin + c);
+    a.phi[c] = phi;
+    most = overlap_of(most, phi);
+  }
+  fold_overlap(sc, most);
 }
 
 // ---------------------------------------------------------------- packing

@@ -931,12 +931,18 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
   // phi of gamma_k; a planar solve that ran out of iterations leaves the
   // gamma_{k-1} of its last residual iteration, as the streaming kernel does
   if (conv || (!k3D && it > 10)) {
+    double most = 0.0;
     for (int x = warp; x < nlv; x += kWarps) {
       each_constraint(vw[x], [&](int c, int s) {
         a.cs.gamma[c] = a.gprev[c];
-        if (conv) a.cs.sd[c] = gg[s].y;
+        if (!conv) return;
+        const double g = gg[s].y;
+        a.cs.sd[c] = g;
+        most = overlap_of(most, g);
       });
     }
+    __syncwarp();
+    fold_overlap(sc, most);
   }
 }
 

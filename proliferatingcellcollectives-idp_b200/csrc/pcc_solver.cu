@@ -23,6 +23,7 @@
 // kernel returns.
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 
 #include "pcc_bbpgd.cuh"
 #include "pcc_kernels.hpp"
@@ -312,10 +313,14 @@ __global__ void __launch_bounds__(kBlock) k_bbpgd(SolverArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) sc->iterations = it;
   if (!*(volatile int*)&sc->converged) return;
   // Returned result (Hard.cpp:170 with BBPGD.cpp:124): gamma_{k-1}, phi(gamma_k).
+  double most = 0.0;
   for (long long c = tid; c < a.m; c += stride) {
+    const double phi = ldcg(a.g[1 - p] + c);
     a.gamma[c] = ldcg(a.gam[p] + c);
-    a.phi[c] = ldcg(a.g[1 - p] + c);
+    a.phi[c] = phi;
+    most = overlap_of(most, phi);
   }
+  fold_overlap(sc, most);
 }
 
 // Cell update after a solve: dC = G U (Physics.cpp:220-265), Euler step and
@@ -355,18 +360,6 @@ __global__ void k_move(CellsView c, long long n, const double* __restrict__ U, c
   c.ldot[i] = ldot[i];
   c.imp[i] = imp[i];
   c.stress[i] = sig[i];
-}
-
-__global__ void k_max_overlap(const double* __restrict__ sd, long long from, long long to,
-                              unsigned long long* __restrict__ dst) {
-  long long c = from + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (c < to) v = sd[c] < 0 ? -sd[c] : 0.0;
-  for (int o = 16; o > 0; o >>= 1) {
-    double w = __shfl_down_sync(0xffffffffu, v, o);
-    v = v < w ? w : v;
-  }
-  if ((threadIdx.x & 31) == 0 && v > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(v));
 }
 
 // x^1.5 correctly rounded in practice: sqrt with its exact residual and the
@@ -703,9 +696,9 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
   // 312 B per constraint and 288 B per cell in FP64; the FP32 operand terms halve
   ctx->bbpgd_pending_bytes = mixed ? 192.0 * (double)m + 144.0 * (double)n : 312.0 * (double)m + 288.0 * (double)n;
   if ((e = cudaMemcpyAsync(ctx->scal_host, ctx->scal.p, kScalarsCopied, cudaMemcpyDeviceToHost, s))) return e;
-  if ((e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s))) return e;
   ctx->bbpgd_pending = true;
   if (defer && !tracing) return cudaSuccess;  // read at the caller's next synchronisation
+  if ((e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s))) return e;
   if ((e = cudaStreamSynchronize(s))) return e;
   const long long it_done = ctx->scal_host->iterations;
   bbpgd_collect(ctx, iterations, residual, status);
@@ -739,6 +732,7 @@ void bbpgd_collect(pcc_ctx* ctx, long long* iterations, double* residual, int* s
   ctx->bbpgd_pending = false;
   *iterations = host.iterations;
   *residual = host.residual;
+  std::memcpy(&ctx->solved_overlap, &host.overlap_bits, sizeof ctx->solved_overlap);
   if (ctx->profiling) {
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
@@ -755,22 +749,11 @@ void bbpgd_collect(pcc_ctx* ctx, long long* iterations, double* residual, int* s
 
 cudaError_t apply_hard_solution(pcc_ctx* ctx, double dt) {
   if (!ctx->n) return cudaSuccess;
+  ctx->box_known = false;
   k_move<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(ctx->cells.view(), (long long)ctx->n, ctx->U.p, ctx->F.p,
                                                        ctx->ldot_new.p, ctx->imp_new.p, ctx->sig.p, dt);
   ctx->launches++;
   return cudaGetLastError();
-}
-
-cudaError_t max_overlap_enqueue(pcc_ctx* ctx, size_t from, size_t to) {
-  cudaStream_t s = ctx->stream;
-  cudaMemsetAsync(&ctx->status->maxold_bits, 0, sizeof(unsigned long long), s);
-  if (to > from) {
-    k_max_overlap<<<grid_for((long long)(to - from)), kBlock, 0, s>>>(ctx->cons.sd.p, (long long)from, (long long)to,
-                                                                     &ctx->status->maxold_bits);
-    ctx->launches++;
-  }
-  return cudaMemcpyAsync(ctx->pinned_ll + kSlotMaxOld, &ctx->status->maxold_bits, sizeof(unsigned long long),
-                         cudaMemcpyDeviceToHost, s);
 }
 
 cudaError_t soft_assemble(pcc_ctx* ctx) {
@@ -796,6 +779,7 @@ cudaError_t soft_forces_and_move(pcc_ctx* ctx, double dt) {
   cudaStream_t s = ctx->stream;
   cudaError_t e;
   const size_t m = ctx->ncons;
+  ctx->box_known = false;
   if ((e = ctx->fel.reserve(m + 1, 0, s))) return e;
   if (m) {
     k_soft_fel<<<grid_for(m), kBlock, 0, s>>>(ctx->cons.view(), (long long)m, ctx->cells.diam.p, ctx->params.kcc,

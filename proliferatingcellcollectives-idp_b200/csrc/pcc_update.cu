@@ -485,6 +485,7 @@ void step_end_collect(pcc_ctx* ctx) {
   const DevStatus& st = *ctx->status_host;
   if (!ctx->params.fixed_dt) adapt_dt(ctx);
   std::memcpy(&ctx->radius, &st.radius_bits, sizeof ctx->radius);
+  ctx->box_known = true;
   ctx->div_next = (size_t)st.divisions;
   ctx->div_known = true;
 }
