@@ -99,8 +99,7 @@ pcc_status cuda_fail(pcc_ctx* ctx, cudaError_t e, const char* where) {
 
 // Reads the device status word; a raised flag becomes an error code.
 pcc_status check_device(pcc_ctx* ctx, const char* where) {
-  cudaError_t e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
-                                  ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(ctx->status_host, ctx->status, kStatusBytes, cudaMemcpyDeviceToHost, ctx->stream);
   if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_fail(ctx, e, where);
   unsigned f = ctx->status_host->flags;
@@ -152,7 +151,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
   ctx->ncons = 0;
   ctx->bbpgd_pending = false;
   CU(reset_ldot(ctx), "reset");
-  CU(mobility(ctx), "mobility");
+  ctx->mobility_known = false;
   // U_ext: Brownian kicks at ReLCP phase 0 only (Hard.cpp:138-143, Physics.cpp:68)
   CU(brownian_draw(ctx), "brownian");
   // reads the scalars of a BBPGD launch after a synchronisation point
@@ -176,7 +175,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
     if (ctx->profiling) cudaEventRecord(ctx->ev[2], ctx->stream);
     CU(detect_contacts(ctx, phase == 0 ? .25 : tol, phase, phase > 0, &added, &ov_new), "detect");
     if (ctx->n == 0) {  // an empty colony's detection did not wait
-      CU(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream), "detect");
+      CU(cudaMemcpyAsync(ctx->status_host, ctx->status, kStatusBytes, cudaMemcpyDeviceToHost, ctx->stream), "detect");
       CU(cudaStreamSynchronize(ctx->stream), "detect");
     }
     pcc_status rc = collect();  // the previous phase's BBPGD, now complete
@@ -187,7 +186,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
       profile_detect(ctx);
       break;
     }
-    CU(build_incidence(ctx), "incidence");
+    CU(build_incidence(ctx, false), "incidence");
     profile_detect(ctx);
     ctx->trace_phase = phase;
     long long it = 0;
@@ -206,7 +205,7 @@ pcc_status solve_hard(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* st, boo
     ++phase;
   }
   if (ctx->bbpgd_pending) {  // the loop ran out of phases right after a solve
-    CU(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream), "bbpgd");
+    CU(cudaMemcpyAsync(ctx->status_host, ctx->status, kStatusBytes, cudaMemcpyDeviceToHost, ctx->stream), "bbpgd");
     CU(cudaStreamSynchronize(ctx->stream), "bbpgd");
     pcc_status rc = collect();
     if (rc) return rc;
@@ -244,7 +243,7 @@ pcc_status solve_soft(pcc_ctx* ctx, double dt, pcc_step_stats* st, bool end_chec
   double max_ov = 0.0;
   if (ctx->profiling) cudaEventRecord(ctx->ev[2], ctx->stream);
   CU(detect_contacts(ctx, 0.0, 0, false, &added, &max_ov), "detect");
-  CU(build_incidence(ctx), "incidence");
+  CU(build_incidence(ctx, true), "incidence");
   profile_detect(ctx);
   CU(soft_forces_and_move(ctx, dt), "soft");
   ctx->uext_active = false;
@@ -370,7 +369,6 @@ pcc_status pcc_create(const pcc_params* params, int device, pcc_ctx** out) {
   if (!e) e = cudaMallocAsync(&ctx->status, sizeof(DevStatus), ctx->stream);
   if (!e) e = cudaMallocHost(&ctx->status_host, sizeof(DevStatus));
   if (!e) e = cudaMallocHost(&ctx->pinned_ll, 64 * sizeof(long long));
-  if (!e) e = cudaMallocHost(&ctx->scal_host, sizeof(SolverScalars));
   if (!e) e = cudaMemsetAsync(ctx->status, 0, sizeof(DevStatus), ctx->stream);
   if (!e && params->capacity_hint > 0) e = ctx->cells.reserve((size_t)params->capacity_hint, 0, ctx->stream);
   if (!e) e = cudaStreamSynchronize(ctx->stream);
@@ -398,7 +396,6 @@ pcc_status pcc_destroy(pcc_ctx* ctx) {
   if (ctx->status) cudaFreeAsync(ctx->status, ctx->stream);
   if (ctx->status_host) cudaFreeHost(ctx->status_host);
   if (ctx->pinned_ll) cudaFreeHost(ctx->pinned_ll);
-  if (ctx->scal_host) cudaFreeHost(ctx->scal_host);
   if (ctx->brown_host) cudaFreeHost(ctx->brown_host);
   cudaStream_t s = ctx->stream;
   delete ctx;  // device buffers are freed on the context's stream
@@ -609,9 +606,9 @@ pcc_status pcc_bbpgd_frozen(pcc_ctx* ctx, double dt, int repeats, long long* ite
   size_t added = 0;
   double mo = 0;
   CU(reset_ldot(ctx), "reset");
-  CU(mobility(ctx), "mobility");
+  ctx->mobility_known = false;
   CU(detect_contacts(ctx, 0.25, 0, false, &added, &mo), "detect");
-  CU(build_incidence(ctx), "incidence");
+  CU(build_incidence(ctx, false), "incidence");
   const size_t m = ctx->ncons;
   DevBuf<double> sd0, g0;
   CU(sd0.reserve(m + 1, 0, s), "frozen");
@@ -662,7 +659,7 @@ pcc_status pcc_soft_forces_frozen(pcc_ctx* ctx, int repeats, float* ms_per_assem
   size_t added = 0;
   double mo = 0;
   CU(detect_contacts(ctx, 0.0, 0, false, &added, &mo), "detect");
-  CU(build_incidence(ctx), "incidence");
+  CU(build_incidence(ctx, true), "incidence");
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);

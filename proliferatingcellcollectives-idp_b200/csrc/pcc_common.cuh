@@ -23,6 +23,28 @@ enum : unsigned {
   kDevErrNan = 1u << 3,        // non-finite values appeared
 };
 
+// Grid barrier + reduction scratch of the persistent solver kernel.
+// The arrival counter sits on a cache line of its own: every block adds to
+// it at every grid barrier, while the release word and the scalars that the
+// blocks read after a release share the next line.
+constexpr int kTakeGroups = 8;
+struct SolverScalars {
+  unsigned long long arrive;     // block arrivals at grid barriers, monotonic within a launch
+  unsigned long long pad0[15];
+  unsigned long long released;   // ordinal of the last barrier whose reduction was published
+  int converged;                 // 1 once the residual test passed
+  int pad;
+  long long iterations;          // BBPGD iteration count at exit
+  double alpha;                  // current step size
+  double residual;               // last evaluated residual
+  double res0;                   // initial residual
+  unsigned long long overlap_bits;  // largest overlap of the constraints after a converged solve
+  // cell-unit counters of the multi-block planar cell pass, two sets used by
+  // alternate iterations, one counter per 128-byte line
+  alignas(128) unsigned long long take[2][kTakeGroups][16];
+};
+static_assert(offsetof(SolverScalars, take) == 256, "counters start on their own line");
+
 struct DevStatus {
   unsigned flags;
   int where;
@@ -40,7 +62,10 @@ struct DevStatus {
   unsigned long long median[2];    // the two middle adaptDt speeds, as ordered keys
   int divisions;                   // of the next step
   int pad2;
+  SolverScalars solver;  // of the last BBPGD launch
 };
+// What the host reads, in one copy: everything but the cell-unit counters.
+constexpr size_t kStatusBytes = offsetof(DevStatus, solver) + offsetof(SolverScalars, take);
 constexpr size_t kDetectBegin = offsetof(DevStatus, max_bits), kDetectBytes = offsetof(DevStatus, radius_bits) - kDetectBegin;
 
 // Cell arrays (device pointers).
@@ -101,6 +126,18 @@ __device__ __forceinline__ void cross3(const double a[3], const double b[3], dou
   r[0] = sub(mul(a[1], b[2]), mul(a[2], b[1]));
   r[1] = sub(mul(a[2], b[0]), mul(a[0], b[2]));
   r[2] = sub(mul(a[0], b[1]), mul(a[1], b[0]));
+}
+
+// Incidence entry k of the unordered lists (2 c + side) and its place in
+// ascending order among its cell's entries.
+__device__ __forceinline__ int entry_place(const int* __restrict__ gi, const int* __restrict__ gj,
+                                           const int* __restrict__ off, const int* __restrict__ raw, size_t k,
+                                           int* at) {
+  const int e = raw[k], p = (e & 1) ? gj[e >> 1] : gi[e >> 1], hi = off[p + 1];
+  int s = off[p];
+  for (int q = s; q < hi; ++q) s += raw[q] < e ? 1 : 0;
+  *at = s;
+  return e;
 }
 
 // Loads that bypass L1: data produced by other blocks of the same

@@ -66,29 +66,6 @@ struct ConsBufs {
   ConsView view();
 };
 
-// Grid barrier + reduction scratch of the persistent solver kernel.
-// The arrival counter sits on a cache line of its own: every block adds to
-// it at every grid barrier, while the release word and the scalars that the
-// blocks read after a release share the next line.
-constexpr int kTakeGroups = 8;
-struct SolverScalars {
-  unsigned long long arrive;     // block arrivals at grid barriers, monotonic within a launch
-  unsigned long long pad0[15];
-  unsigned long long released;   // ordinal of the last barrier whose reduction was published
-  int converged;                 // 1 once the residual test passed
-  int pad;
-  long long iterations;          // BBPGD iteration count at exit
-  double alpha;                  // current step size
-  double residual;               // last evaluated residual
-  double res0;                   // initial residual
-  // cell-unit counters of the multi-block planar cell pass, two sets used by
-  // alternate iterations, one counter per 128-byte line; not copied back
-  unsigned long long overlap_bits;  // largest overlap of the constraints after a converged solve
-  alignas(128) unsigned long long take[2][kTakeGroups][16];
-};
-constexpr size_t kScalarsCopied = offsetof(SolverScalars, take);
-static_assert(offsetof(SolverScalars, take) == 256, "counters start on their own line");
-
 }  // namespace pcc
 
 struct pcc_vtk_writer_state;
@@ -109,7 +86,7 @@ struct pcc_ctx {
   pcc::ConsBufs cons;
 
   // detection scratch
-  pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_cursor, bin_raw, bin_cells, cand_cnt, cand_off;
+  pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_raw, bin_cells, cand_cnt, cand_off;
   pcc::DevBuf<double> pk;  // packed per-cell geometry in bin order
   pcc::DevBuf<int> ghost;
   bool box_known = false;  // radius bounds the centres of the resident cells
@@ -122,13 +99,12 @@ struct pcc_ctx {
   double list_tol = 0.0;
 
   // incidence CSR (cell -> constraint sides)
-  pcc::DevBuf<int> inc_cnt, inc_off, inc_ent;
+  pcc::DevBuf<int> inc_cnt, inc_off, inc_cur, inc_raw, inc_ent;  // counts run over the phases of a step
 
   // solver scratch
   pcc::DevBuf<double> gam_a, gam_b, g_a, g_b, gam_old;
   pcc::DevBuf<double> U, dldot, F, sig, ldot_new, imp_new, Mlin, Mrot, ldot_prev;
   pcc::DevBuf<double> partials;
-  pcc::DevBuf<pcc::SolverScalars> scal;
   pcc::DevBuf<double> fel;  // soft: Hertz force magnitude per contact
   // packed operands of the planar solver
   pcc::DevBuf<int2> p_ij;
@@ -158,9 +134,9 @@ struct pcc_ctx {
   pcc::DevBuf<double> red;  // small reductions
 
   // host round trips: values enqueued for the next synchronisation point
-  pcc::SolverScalars* scal_host = nullptr;  // pinned: BBPGD scalars of a launch not yet read
-  bool bbpgd_pending = false;               // a BBPGD launch whose scalars are still on their way
+  bool bbpgd_pending = false;               // a BBPGD launch whose scalars are not read yet
   double bbpgd_pending_bytes = 0.0;         // its algorithmic bytes per iteration
+  bool mobility_known = false;              // Mlin / Mrot describe the resident cells
   double solved_overlap = 0.0;              // largest overlap that the last solve left
   bool div_known = false;                   // div_flag / div_off / div_next describe the resident cells
   size_t div_next = 0;                      // divisions the next step commits

@@ -13,8 +13,9 @@ constexpr int kSlotDivs = 11;    // divisions of the next step
 
 // ---- pcc_scan_sort.cu
 // out[i] = sum in[0..i-1] for i in [0, n]; out has n+1 entries.  The sum of
-// all goes to *total too (a device address) if given.
-cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total = nullptr);
+// all goes to *total too (a device address) if given, and entries [0, n) to
+// copy.
+cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total = nullptr, int* copy = nullptr);
 // Stable ascending sort of (keys, vals) by the low `bits` bits of keys;
 // keys/vals are sorted in place (scratch from ctx).
 cudaError_t radix_sort_pairs(pcc_ctx* ctx, unsigned long long* keys, int* vals, size_t n, int bits);
@@ -27,17 +28,22 @@ cudaError_t radix_sort_pairs(pcc_ctx* ctx, unsigned long long* keys, int* vals, 
 // pass it only when the cells changed by constraint motion alone since.
 cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, size_t* added,
                             double* max_overlap_new);
-// Cell -> incident constraint sides, ascending constraint index, for ctx->ncons.
-cudaError_t build_incidence(pcc_ctx* ctx);
+// Cell -> incident constraint sides for ctx->ncons: the offsets and, with
+// order, the entries in ascending constraint order (inc_ent); without, the
+// entries of each cell in no order (inc_raw), for order_incidence or a solver
+// that orders them as it packs them.
+cudaError_t build_incidence(pcc_ctx* ctx, bool order);
+cudaError_t order_incidence(pcc_ctx* ctx);
 
 // ---- pcc_solver.cu
 // Draws the Brownian U_ext of every cell (temperature > 0) from the context's
 // generator and sets ctx->uext_active; a no-op at temperature 0.
 cudaError_t brownian_draw(pcc_ctx* ctx);
 // One BBPGD solve on the current constraint set (hard model).  With defer,
-// only launches it and enqueues the copy of its scalars (ctx->bbpgd_pending);
+// only launches it (ctx->bbpgd_pending);
 // bbpgd_collect reads them after the caller's next synchronisation that also
-// copied the device status.  It sets ctx->solved_overlap.
+// copied the device status.  It sets ctx->solved_overlap.  Expects the
+// incidence without order.
 cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* residual, int* status,
                         bool defer = false);
 void bbpgd_collect(pcc_ctx* ctx, long long* iterations, double* residual, int* status);
@@ -64,7 +70,8 @@ long long planar_chunks(size_t m);
 cudaError_t planar_bbpgd(pcc_ctx* ctx, double dt, bool mixed, const PlanarTrace& tr, int* kind);
 
 // ---- pcc_resident.cu
-// Launches the on-chip BBPGD solve if the constraint set fits it (*taken);
+// Launches the on-chip BBPGD solve (and the ordering of the incidence lists) if
+// the constraint set fits it (*taken);
 // full: six D components.  *kind as for planar_bbpgd.
 cudaError_t resident_bbpgd(pcc_ctx* ctx, double dt, bool full, bool mixed, bool* taken, int* kind);
 
@@ -86,6 +93,7 @@ void step_end_collect(pcc_ctx* ctx);
 // Sort cells by x (stable) and renumber.
 cudaError_t sort_cells_by_x(pcc_ctx* ctx);
 cudaError_t colony_radius(pcc_ctx* ctx, double* out);
+// Per-cell mobilities for the streaming solvers, unless ctx->mobility_known.
 cudaError_t mobility(pcc_ctx* ctx);
 
 // ---- pcc_vtk.cu

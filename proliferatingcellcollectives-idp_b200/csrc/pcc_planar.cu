@@ -557,21 +557,24 @@ __global__ void k_pack_planar_cons(ConsView cs, long long m, int2* __restrict__ 
   gg0[c] = make_double2(cs.gamma[c], 0.0);
 }
 
-// Per incidence entry: its side's D row and the constraint's gamma_old.
+// Per incidence entry, from the unordered lists to its place in the ordered
+// ones: the entry, its side's D row and the constraint's gamma_old.
 template <class Real>
-__global__ void k_pack_planar_inc(ConsView cs, const int* __restrict__ inc_ent, long long ne,
-                                  typename PT<Real>::V4* __restrict__ inc, double* __restrict__ gold) {
+__global__ void k_pack_planar_inc(ConsView cs, const int* __restrict__ off, const int* __restrict__ raw, size_t ne,
+                                  int* __restrict__ ents, typename PT<Real>::V4* __restrict__ inc,
+                                  double* __restrict__ gold) {
   using V4 = typename PT<Real>::V4;
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ne) return;
-  const int ent = inc_ent[k];
+  int at;
+  const int ent = entry_place(cs.gi, cs.gj, off, raw, k, &at);
   const long long c = ent >> 1;
-  const int side = ent & 1;
-  if (side == 0)
-    inc[k] = mk4<V4>(cs.nx[c], cs.ny[c], cs.tiz[c], cs.si[c]);
+  ents[at] = ent;
+  if ((ent & 1) == 0)
+    inc[at] = mk4<V4>(cs.nx[c], cs.ny[c], cs.tiz[c], cs.si[c]);
   else
-    inc[k] = mk4<V4>(-cs.nx[c], -cs.ny[c], cs.tjz[c], cs.sj[c]);
-  gold[k] = cs.gamma[c];
+    inc[at] = mk4<V4>(-cs.nx[c], -cs.ny[c], cs.tjz[c], cs.sj[c]);
+  gold[at] = cs.gamma[c];
 }
 
 template <class Real>
@@ -625,8 +628,8 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
   if (m) {
     k_pack_planar_cons<Real><<<grid_for((long long)m), kBlock, 0, s>>>(cv, (long long)m, ctx->p_ij.p, B::nn(ctx).p,
                                                                        B::tt(ctx).p, B::ss(ctx).p, ctx->p_gg.p);
-    k_pack_planar_inc<Real><<<grid_for((long long)ne), kBlock, 0, s>>>(cv, ctx->inc_ent.p, (long long)ne,
-                                                                       B::inc(ctx).p, ctx->p_gold.p);
+    k_pack_planar_inc<Real><<<grid_for((long long)ne), kBlock, 0, s>>>(
+        cv, ctx->inc_off.p, ctx->inc_raw.p, ne, ctx->inc_ent.p, B::inc(ctx).p, ctx->p_gold.p);
     ctx->launches += 2;
   }
   if (n) {
@@ -664,7 +667,7 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
   a.partials = reinterpret_cast<double4*>(ctx->partials.p);
   a.nchunks = nchunks;
   a.ent = ctx->inc_ent.p;
-  a.sc = ctx->scal.p;
+  a.sc = &ctx->status->solver;
   a.st_err = ctx->status;
   a.trace = tr.trace;
   a.tr_part = tr.tr_part;

@@ -85,13 +85,13 @@ struct ResArgs {
   long long m, n;
   ConsView cs;
   const int *inc_off, *inc_ent;
-  const double *Mlin, *Mrot, *len, *ldot_prev;
+  const double *len, *ldot_prev;
   const double* uext;       // rotational U_ext, 3 per cell; null: zero
   double2* gg;              // grid form: (gamma, g) of the last iteration
   double* gprev;            // gamma_{k-1} of the last residual iteration
   void* u;                  // grid form: velocity rows
   double *U, *F, *sig, *ldot, *imp;
-  double dt, lambda, tau, tol;
+  double dt, lambda, tau, xi, tol;
   long long max_it;
   double* partials;         // grid form: value-major, one per chunk
   long long nchunks;
@@ -292,9 +292,10 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
   const int ngroups = (ncell + kGroup - 1) / kGroup;
   for (int i = t; i <= ncell; i += T) soff[i] = a.inc_off[cb + i] - eb;
   for (int i = t; i < ncell; i += T) {
-    cellc[4 * i] = (Real)a.Mlin[cb + i];
-    cellc[4 * i + 1] = (Real)a.Mrot[cb + i];
-    cellc[4 * i + 2] = (Real)a.len[cb + i];
+    const double l = a.len[cb + i];
+    cellc[4 * i] = (Real)dvd(1.0, mul(l, a.xi));  // mobilities (Physics.cpp:192-218)
+    cellc[4 * i + 1] = (Real)dvd(12.0, mul(mul(mul(l, l), l), a.xi));
+    cellc[4 * i + 2] = (Real)l;
     cellc[4 * i + 3] = (Real)a.ldot_prev[cb + i];
     if constexpr (kCluster) umask[i] = 0;
   }
@@ -881,6 +882,7 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
 
   // ---------------------------------------------------------------- solve
   const bool recorder = rank == 0 && t == 0;
+  if (recorder) sc->overlap_bits = 0;  // the barriers of an iteration order it before the sums at the end
   double v[4] = {0, 0, 0, 0};
   if constexpr (kCluster) meet();
   else __syncthreads();
@@ -1055,8 +1057,6 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
   a.cs = ctx->cons.view();
   a.inc_off = ctx->inc_off.p;
   a.inc_ent = ctx->inc_ent.p;
-  a.Mlin = ctx->Mlin.p;
-  a.Mrot = ctx->Mrot.p;
   a.len = ctx->cells.len.p;
   a.ldot_prev = ctx->cells.ldot.p;
   a.uext = ctx->uext_active ? ctx->uext.p : nullptr;
@@ -1071,6 +1071,7 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
   a.dt = dt;
   a.lambda = ctx->params.lambda;
   a.tau = ctx->params.tau;
+  a.xi = ctx->params.xi;
   a.tol = ctx->params.tolerance;
   a.max_it = ctx->params.max_bbpgd_iterations;
   a.partials = ctx->partials.p;
@@ -1083,8 +1084,11 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
   a.cells_max = sh.cells_max;
   a.cap = sh.cap;
   a.kappa = sh.kappa;
-  a.sc = ctx->scal.p;
+  a.sc = &ctx->status->solver;
   a.st = ctx->status;
+  if ((e = order_incidence(ctx))) return e;
+  // the grid form's barrier counts from zero; a cluster clears what it adds to
+  if (!cluster) cudaMemsetAsync(a.sc, 0, sizeof(SolverScalars), s);
   void* args[] = {&a};
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], s);
   cudaLaunchConfig_t cfg = {};

@@ -10,7 +10,7 @@ namespace {
 constexpr int kScanItems = 8;                      // items per thread
 constexpr int kScanTile = kBlock * kScanItems;     // 2048 per block
 constexpr int kOneThreads = 1024;                  // one-block scan
-constexpr long long kOneMost = 4LL * kOneThreads * kScanItems;
+constexpr long long kOneMost = 2LL * kOneThreads * kScanItems;
 constexpr int kSumsMost = 4096;                    // block sums that every block adds up by itself
 
 // Warp-shuffle scan of one value per thread across a block of kThreads.
@@ -42,10 +42,10 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* smem, int* total
 }
 
 // Scan of a short array by one block: one launch instead of the two below
-// (three before); bound by launch latency.  Up to 32,768 items, four rounds
-// of the block, beyond which the rounds take longer than the second launch.
+// (three before); bound by launch latency.  Up to 16,384 items, two rounds
+// of the block (5 us); three rounds took 12 us, longer than two launches.
 __global__ void __launch_bounds__(kOneThreads) k_scan_one(const int* __restrict__ in, int n, int* __restrict__ out,
-                                                          int* __restrict__ total) {
+                                                          int* __restrict__ total, int* __restrict__ copy) {
   __shared__ int sm[kOneThreads / 32];
   int carry = 0;
   for (int base = 0; base < n; base += kOneThreads * kScanItems) {
@@ -60,7 +60,10 @@ __global__ void __launch_bounds__(kOneThreads) k_scan_one(const int* __restrict_
     int ex = carry + block_exclusive_scan<kOneThreads>(s, sm, &tot);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-      if (b + k < n) out[b + k] = ex;
+      if (b + k < n) {
+        out[b + k] = ex;
+        if (copy) copy[b + k] = ex;
+      }
       ex += v[k];
     }
     carry += tot;
@@ -99,7 +102,7 @@ __global__ void k_scan_blocks(int* bsum, int nb) {
 // scanned: bsum holds the blocks' offsets already (very long arrays);
 // otherwise each block adds up the sums before it.
 __global__ void k_scan_apply(const int* __restrict__ in, size_t n, const int* __restrict__ bsum, bool scanned,
-                             int* __restrict__ out, int* __restrict__ total) {
+                             int* __restrict__ out, int* __restrict__ total, int* __restrict__ copy) {
   __shared__ int sm[kBlock / 32];
   int before = 0;
   if (scanned) {
@@ -121,7 +124,10 @@ __global__ void k_scan_apply(const int* __restrict__ in, size_t n, const int* __
   int ex = block_exclusive_scan<kBlock>(s, sm, &tot) + before;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    if (base + k < n) out[base + k] = ex;
+    if (base + k < n) {
+      out[base + k] = ex;
+      if (copy) copy[base + k] = ex;
+    }
     ex += v[k];
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
@@ -201,10 +207,10 @@ __global__ void k_radix_scatter(const unsigned long long* __restrict__ keys, con
 
 }  // namespace
 
-cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total) {
+cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int* total, int* copy) {
   cudaStream_t s = ctx->stream;
   if ((long long)n <= kOneMost) {
-    k_scan_one<<<1, kOneThreads, 0, s>>>(in, (int)n, out, total);
+    k_scan_one<<<1, kOneThreads, 0, s>>>(in, (int)n, out, total, copy);
     ctx->launches++;
     return cudaGetLastError();
   }
@@ -215,7 +221,7 @@ cudaError_t exclusive_scan(pcc_ctx* ctx, const int* in, int* out, size_t n, int*
   const bool scanned = nb > (size_t)kSumsMost;
   k_scan_reduce<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum);
   if (scanned) k_scan_blocks<<<1, kBlock, 0, s>>>(bsum, (int)nb);
-  k_scan_apply<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum, scanned, out, total);
+  k_scan_apply<<<(unsigned)nb, kBlock, 0, s>>>(in, n, bsum, scanned, out, total, copy);
   ctx->launches += scanned ? 3 : 2;
   return cudaGetLastError();
 }

@@ -562,6 +562,8 @@ cudaError_t brownian_draw(pcc_ctx* ctx) {
 cudaError_t mobility(pcc_ctx* ctx) {
   cudaStream_t s = ctx->stream;
   cudaError_t e;
+  if (ctx->mobility_known) return cudaSuccess;
+  ctx->mobility_known = true;
   if ((e = ctx->Mlin.reserve(ctx->n + 1, 0, s))) return e;
   if ((e = ctx->Mrot.reserve(ctx->n + 1, 0, s))) return e;
   if (ctx->n) {
@@ -581,8 +583,7 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
   if ((e = ctx->U.reserve(6 * nn, 0, s)) || (e = ctx->dldot.reserve(nn, 0, s)) || (e = ctx->F.reserve(6 * nn, 0, s)) ||
       (e = ctx->sig.reserve(nn, 0, s)) || (e = ctx->ldot_new.reserve(nn, 0, s)) || (e = ctx->imp_new.reserve(nn, 0, s)))
     return e;
-  if ((e = ctx->scal.reserve(1, 0, s))) return e;
-  cudaMemsetAsync(ctx->scal.p, 0, sizeof(SolverScalars), s);
+  SolverScalars* sc = &ctx->status->solver;
   const long long nchunks = chunk_count((long long)m);  // the FP64 planar kernel's chunks
   const bool tracing = ctx->trace_active;
   long long trace_cap = 0;
@@ -602,12 +603,17 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
   int kind = 0;
   bool on_chip = false;
   if (!tracing && (e = resident_bbpgd(ctx, dt, !planar, mixed, &on_chip, &kind))) return e;
+  if (!on_chip) {
+    cudaMemsetAsync(sc, 0, sizeof(SolverScalars), s);
+    if ((e = mobility(ctx))) return e;
+  }
   if (on_chip) {
     // launched
   } else if (planar) {  // records ev[0] itself, after packing its operands
     const PlanarTrace tr{trace, ctx->tr_part.p, ctx->trace_dev.p, trace_cap};
     e = planar_bbpgd(ctx, dt, mixed, tr, &kind);
   } else {
+    if ((e = order_incidence(ctx))) return e;
     if ((e = ctx->gam_a.reserve(mm, 0, s)) || (e = ctx->gam_b.reserve(mm, 0, s)) || (e = ctx->g_a.reserve(mm, 0, s)) ||
         (e = ctx->g_b.reserve(mm, 0, s)))
       return e;
@@ -655,7 +661,7 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
     a.max_it = ctx->params.max_bbpgd_iterations;
     a.partials = ctx->partials.p;
     a.nchunks = nchunks;
-    a.sc = ctx->scal.p;
+    a.sc = sc;
     a.st = ctx->status;
     a.trace = trace;
     a.tr_part = ctx->tr_part.p;
@@ -695,12 +701,11 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], s);
   // 312 B per constraint and 288 B per cell in FP64; the FP32 operand terms halve
   ctx->bbpgd_pending_bytes = mixed ? 192.0 * (double)m + 144.0 * (double)n : 312.0 * (double)m + 288.0 * (double)n;
-  if ((e = cudaMemcpyAsync(ctx->scal_host, ctx->scal.p, kScalarsCopied, cudaMemcpyDeviceToHost, s))) return e;
   ctx->bbpgd_pending = true;
   if (defer && !tracing) return cudaSuccess;  // read at the caller's next synchronisation
-  if ((e = cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s))) return e;
+  if ((e = cudaMemcpyAsync(ctx->status_host, ctx->status, kStatusBytes, cudaMemcpyDeviceToHost, s))) return e;
   if ((e = cudaStreamSynchronize(s))) return e;
-  const long long it_done = ctx->scal_host->iterations;
+  const long long it_done = ctx->status_host->solver.iterations;
   bbpgd_collect(ctx, iterations, residual, status);
   if (tracing) {
     // records 0 .. the last iteration run (BBPGD.cpp:55-81)
@@ -728,7 +733,7 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
 }
 
 void bbpgd_collect(pcc_ctx* ctx, long long* iterations, double* residual, int* status) {
-  const SolverScalars& host = *ctx->scal_host;
+  const SolverScalars& host = ctx->status_host->solver;
   ctx->bbpgd_pending = false;
   *iterations = host.iterations;
   *residual = host.residual;

@@ -451,7 +451,7 @@ cudaError_t step_end_enqueue(pcc_ctx* ctx) {
         return e;
     }
   }
-  return cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
+  return cudaMemcpyAsync(ctx->status_host, ctx->status, kStatusBytes, cudaMemcpyDeviceToHost, s);
 }
 
 // Domain::adaptDt (spatial/Domain.cpp:69-118): median of |v| + ldot (for an
