@@ -1047,7 +1047,8 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
       cluster = shape_for<Real, k3D, true>(m, n, nchunks, ctx->trace_phase + 1, nb, &sh);
     }
   }
-  if (!cluster && !shape_for<Real, k3D, false>(m, n, nchunks, 1, ctx->num_sms, &sh)) return cudaSuccess;
+  const int blocks = (int)(nchunks < ctx->num_sms ? nchunks : ctx->num_sms);
+  if (!cluster && !shape_for<Real, k3D, false>(m, n, nchunks, 1, blocks, &sh)) return cudaSuccess;
   if ((e = ctx->p_gg.reserve(m + 1, 0, s)) || (e = ctx->p_phin.reserve(m + 1, 0, s)) ||
       (e = ctx->partials.reserve(4 * (nchunks + 1), 0, s)) || (e = ctx->p_u.reserve(2 * (n + 1), 0, s)))
     return e;
