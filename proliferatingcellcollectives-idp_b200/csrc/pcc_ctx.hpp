@@ -85,6 +85,8 @@ struct pcc_ctx {
   size_t ncons = 0;
   pcc::ConsBufs cons;
 
+  pcc::DevBuf<double> interleaved;  // vectors of the contacts on their way to the host
+
   // detection scratch
   pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_raw, bin_cells, cand_cnt, cand_off;
   pcc::DevBuf<double> pk;  // packed per-cell geometry in bin order

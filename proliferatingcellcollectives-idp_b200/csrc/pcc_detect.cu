@@ -710,7 +710,22 @@ __global__ void k_inc_order(const int* __restrict__ gi, const int* __restrict__ 
   ent[at] = e;
 }
 
+__global__ void k_interleave3(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                              size_t n, double* __restrict__ out) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // one value: the writes are consecutive
+  if (t >= 3 * n) return;
+  const size_t k = t / 3;
+  const int d = (int)(t - 3 * k);
+  out[t] = d == 0 ? x[k] : d == 1 ? y[k] : z[k];
+}
+
 }  // namespace
+
+cudaError_t interleave3(pcc_ctx* ctx, const double* x, const double* y, const double* z, size_t n) {
+  k_interleave3<<<grid_for((long long)(3 * n)), kBlock, 0, ctx->stream>>>(x, y, z, n, ctx->interleaved.p);
+  ctx->launches++;
+  return cudaGetLastError();
+}
 
 // Grid of the bins of every centre within `r` of the origin, if it is not too
 // large for the colony (a long chain's box would be mostly empty); at z the
