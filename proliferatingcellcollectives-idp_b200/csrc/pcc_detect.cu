@@ -374,10 +374,10 @@ __device__ __forceinline__ bool rough_pass(const double4& a0, const double4& b0,
 // prefilter.  With full == false only the separation is computed.
 __device__ __forceinline__ bool pair_geom(const double* __restrict__ A, const double* __restrict__ B, double tol,
                                           bool full, PairGeom* o) {
-  const double4 a1 = *reinterpret_cast<const double4*>(A + 4);
-  const double4 a2 = *reinterpret_cast<const double4*>(A + 8);
-  const double4 b1 = *reinterpret_cast<const double4*>(B + 4);
-  const double4 b2 = *reinterpret_cast<const double4*>(B + 8);
+  const double4 a1 = ld256(reinterpret_cast<const double4*>(A + 4));
+  const double4 a2 = ld256(reinterpret_cast<const double4*>(A + 8));
+  const double4 b1 = ld256(reinterpret_cast<const double4*>(B + 4));
+  const double4 b2 = ld256(reinterpret_cast<const double4*>(B + 8));
   const double P0[3] = {a1.x, a1.y, a1.z}, P1[3] = {a2.x, a2.y, a2.z};
   const double Q0[3] = {b1.x, b1.y, b1.z}, Q1[3] = {b2.x, b2.y, b2.z};
   double c0[3], c1[3], dist;
@@ -401,10 +401,10 @@ __device__ __forceinline__ bool pair_geom(const double* __restrict__ A, const do
     o->n[1] = 0.0;
     o->n[2] = 0.0;
   }
-  const double4 a0 = *reinterpret_cast<const double4*>(A);
-  const double4 b0 = *reinterpret_cast<const double4*>(B);
-  const double4 a3 = *reinterpret_cast<const double4*>(A + 12);
-  const double4 b3 = *reinterpret_cast<const double4*>(B + 12);
+  const double4 a0 = ld256(reinterpret_cast<const double4*>(A));
+  const double4 b0 = ld256(reinterpret_cast<const double4*>(B));
+  const double4 a3 = ld256(reinterpret_cast<const double4*>(A + 12));
+  const double4 b3 = ld256(reinterpret_cast<const double4*>(B + 12));
   const double ta[3] = {a3.x, a3.y, a3.z}, tb[3] = {b3.x, b3.y, b3.z};
   const double nn[3] = {-o->n[0], -o->n[1], -o->n[2]};
   o->si = mul(0.5, fabs(dot3(o->n, ta)));
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_count(const double* __restrict_
   if (s < n) {
     const double* A = pk + s * kPack;
     const int a = (int)A[11];
-    const double4 a0 = *reinterpret_cast<const double4*>(A);
+    const double4 a0 = ld256(reinterpret_cast<const double4*>(A));
     if (l < 3) xref[3 * (size_t)a + l] = A[l];
     const int bx = binxyz[3 * (size_t)a] - g.mx, by = binxyz[3 * (size_t)a + 1] - g.my,
               bz = binxyz[3 * (size_t)a + 2] - g.mz;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_count(const double* __restrict_
           const int s2 = s0 + l;
           const double* B = pk + (size_t)s2 * kPack;
           bool in = false;
-          if (s2 < hi && (int)B[11] > a) in = rough_pass(a0, *reinterpret_cast<const double4*>(B), tol_list);
+          if (s2 < hi && (int)B[11] > a) in = rough_pass(a0, ld256(reinterpret_cast<const double4*>(B)), tol_list);
           const unsigned hits = __ballot_sync(group, in) >> shift & kOnes;
           const int at = nl + __popc(hits & ((1u << l) - 1u));
           nl += __popc(hits);
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_count(const double* __restrict_
           if (at < kList) {
             list[at] = s2;
             plist[(size_t)a * kList + at] = s2;
-          } else if (!(tol < tol_list) || rough_pass(a0, *reinterpret_cast<const double4*>(B), tol)) {
+          } else if (!(tol < tol_list) || rough_pass(a0, ld256(reinterpret_cast<const double4*>(B)), tol)) {
             test(B, (int)B[11]);  // no room in the list
           }
         }
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_count(const double* __restrict_
     const int listed = nl < kList ? nl : kList;
     for (int k = l; k < listed; k += kPairLanes) {
       const double* B = pk + (size_t)list[k] * kPack;
-      if (tol < tol_list && !rough_pass(a0, *reinterpret_cast<const double4*>(B), tol)) continue;
+      if (tol < tol_list && !rough_pass(a0, ld256(reinterpret_cast<const double4*>(B)), tol)) continue;
       test(B, (int)B[11]);
     }
 #pragma unroll
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kBlock) k_list_pass(
   double maxov = 0.0;
   if (a < n) {
     const double* A = pk + (size_t)slot_of[a] * kPack;
-    const double4 a0 = *reinterpret_cast<const double4*>(A);
+    const double4 a0 = ld256(reinterpret_cast<const double4*>(A));
     const int ga = A[15] != 0.0;
     const int nl = min(plist_n[a], kList);  // lists in use never overflowed
     int bxa = 0, bya = 0, bza = 0;
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kBlock) k_list_pass(
                     ez = binxyz[3 * (size_t)b + 2] - bza;
           pass = ex >= -1 && ex <= 1 && ey >= -1 && ey <= 1 && ez >= -1 && ez <= 1;
         }
-        pass = pass && rough_pass(a0, *reinterpret_cast<const double4*>(B), tol);
+        pass = pass && rough_pass(a0, ld256(reinterpret_cast<const double4*>(B)), tol);
         pass = pass && pair_geom(A, B, tol, kEmit, &pg);
         gb = pass && B[15] != 0.0;
       }
@@ -665,7 +665,7 @@ __global__ void k_stencil_emit(const double* __restrict__ pk, const int* __restr
   if (s >= n) return;
   const double* A = pk + s * kPack;
   const int a = (int)A[11];
-  const double4 a0 = *reinterpret_cast<const double4*>(A);
+  const double4 a0 = ld256(reinterpret_cast<const double4*>(A));
   const int bx = binxyz[3 * (size_t)a] - g.mx, by = binxyz[3 * (size_t)a + 1] - g.my,
             bz = binxyz[3 * (size_t)a + 2] - g.mz;
   size_t w = base + (size_t)off[a];
@@ -677,7 +677,7 @@ __global__ void k_stencil_emit(const double* __restrict__ pk, const int* __restr
         const double* B = pk + (size_t)s2 * kPack;
         const int b = (int)B[11];
         if (b <= a) continue;
-        const double4 b0 = *reinterpret_cast<const double4*>(B);
+        const double4 b0 = ld256(reinterpret_cast<const double4*>(B));
         if (!rough_pass(a0, b0, tol)) continue;
         PairGeom pg;
         if (!pair_geom(A, B, tol, true, &pg)) continue;

@@ -58,7 +58,8 @@ namespace {
 
 // Entries of a lane whose loads are in flight together in the cell pass, and
 // co-resident blocks per SM of the multi-block form: with four entries ahead
-// three blocks fit the registers.  Measured, us per iteration, 44,700 cells
+// three blocks fit the registers.  Measured with two 16-byte loads per FP64 row
+// (one 32-byte load now: 20.4 and 110.5), us per iteration, 44,700 cells
 // FP64 / mixed and 302,172 cells FP64 / mixed: one ahead, four blocks 24.0 / - /
 // - / 93.2; two, four 26.2 / 18.7 / 145.8 / 89.5; four, three 22.7 / 17.7 /
 // 110.8 / 91.1; four, two 21.4 / 17.8 / 114.8 / 100.5.
@@ -201,7 +202,7 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
     }
 #pragma unroll
     for (int q = 0; q < kN; ++q) {
-      d[q] = a.inc[k + q * kLanes];
+      d[q] = ld256(a.inc + k + q * kLanes);
       go[q] = a.gold[k + q * kLanes];
     }
     if (mode != 0) {
@@ -344,8 +345,8 @@ __device__ __forceinline__ double planar_grad(const PArgs<Real>& a, long long c)
   const auto n = a.nn[c];
   const auto t = a.tt[c];
   const auto s = a.ss[c];
-  const auto ui = ldcg(a.u + ij.x);
-  const auto uj = ldcg(a.u + ij.y);
+  const auto ui = ldcg256(a.u + ij.x);
+  const auto uj = ldcg256(a.u + ij.y);
   if constexpr (sizeof(Real) == 8) {
     double pd = 0.0;
     pd = add(pd, mul(n.x, ui.x));

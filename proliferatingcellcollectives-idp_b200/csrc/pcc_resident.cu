@@ -700,10 +700,17 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
   };
 
   auto load_u = [&](int p, Real u[F::kU]) {
+    constexpr int kStep = kCluster || !kF64 ? kPiece : 4;
 #pragma unroll
-    for (int q = 0; q < F::kU; q += kPiece) {
+    for (int q = 0; q < F::kU; q += kStep) {
       if constexpr (kCluster) {
         *reinterpret_cast<int4*>(u + q) = *reinterpret_cast<const int4*>(us + (size_t)F::kU * p + q);
+      } else if constexpr (kF64) {
+        const double4 w = ldcg256(reinterpret_cast<const double4*>(a.u) + ((size_t)F::kU * p + q) / 4);
+        u[q] = w.x;
+        u[q + 1] = w.y;
+        u[q + 2] = w.z;
+        u[q + 3] = w.w;
       } else {
         *reinterpret_cast<int4*>(u + q) =
             __ldcg(reinterpret_cast<const int4*>(reinterpret_cast<const Real*>(a.u) + (size_t)F::kU * p + q));
