@@ -155,25 +155,33 @@ __device__ __forceinline__ double4 ldcg<double4>(const double4* p) {
 
 // One 32-byte load of a row of four, 32-byte aligned (rows of a buffer of the
 // context): lanes that read scattered or strided rows cost L1 one lookup per
-// row, not two.  ld256 is for rows that the kernel does not write, ldcg256 for
-// rows that other blocks of it wrote before a grid barrier.  Streaming FP64
-// BBPGD, per iteration: 362,000 constraints (in L2) 22.8 -> 20.4 us, 2.4 M
-// (from DRAM) 114.4 -> 110.5; on-chip grid form, FP64, 76,000: 9.65 -> 9.05.
+// row, not two.  ld256 is for rows that the kernel does not write, ld256w for
+// rows that other blocks of it wrote before a grid barrier (not moved across
+// it).  Streaming FP64 BBPGD, per iteration: 362,000 constraints (in L2) 22.8
+// -> 20.4 us, 2.4 M (from DRAM) 114.4 -> 110.5; on-chip grid form, FP64,
+// 76,000: 9.65 -> 9.05.
+//
+// ld256w and the solvers' other reads of (gamma, g) and velocity rows may stay
+// in L1: a grid barrier is a release by every block and an acquire by every
+// block, which drops the L1 lines of the SM, and the compiler keeps loads on
+// their side of it.  Neighbouring constraints share cells, so a row is read
+// again by the same SM: 20.4 -> 19.9 us per iteration (mixed 17.5 -> 16.5) and
+// 109.5 -> 105.3 (91.0 -> 86.9) against loads that bypass L1.
 __device__ __forceinline__ double4 ld256(const double4* p) {
   double4 r;
   asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
   return r;
 }
 __device__ __forceinline__ float4 ld256(const float4* p) { return *p; }  // 16 bytes: one load as it is
-__device__ __forceinline__ double4 ldcg256(const double4* p) {
+__device__ __forceinline__ double4 ld256w(const double4* p) {
   double4 r;
-  asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
                : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w)
                : "l"(p)
                : "memory");
   return r;
 }
-__device__ __forceinline__ float4 ldcg256(const float4* p) { return __ldcg(p); }
+__device__ __forceinline__ float4 ld256w(const float4* p) { return *p; }
 
 __device__ __forceinline__ void raise_error(DevStatus* st, unsigned flag, int where) {
   atomicOr(&st->flags, flag);

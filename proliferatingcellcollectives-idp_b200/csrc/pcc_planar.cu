@@ -58,8 +58,9 @@ namespace {
 
 // Entries of a lane whose loads are in flight together in the cell pass, and
 // co-resident blocks per SM of the multi-block form: with four entries ahead
-// three blocks fit the registers.  Measured with two 16-byte loads per FP64 row
-// (one 32-byte load now: 20.4 and 110.5), us per iteration, 44,700 cells
+// three blocks fit the registers (a few spilled bytes cost a quarter: loop
+// counters are 32-bit).  Measured before the 32-byte and L1-resident row loads
+// (19.9 / 16.3 / 106 / 86 now), us per iteration, 44,700 cells
 // FP64 / mixed and 302,172 cells FP64 / mixed: one ahead, four blocks 24.0 / - /
 // - / 93.2; two, four 26.2 / 18.7 / 145.8 / 89.5; four, three 22.7 / 17.7 /
 // 110.8 / 91.1; four, two 21.4 / 17.8 / 114.8 / 100.5.
@@ -168,7 +169,7 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
   using V4 = typename PT<Real>::V4;
   constexpr bool kF64 = sizeof(Real) == 8;
   const int lane = threadIdx.x & 31, gl = lane % kLanes;
-  constexpr long long kCellsPerWarp = 32 / kLanes;
+  constexpr int kCellsPerWarp = 32 / kLanes;
   auto accumulate = [&](CellAcc<Real>& A, const V4& d, double go, double gc) {
     const double diff = sub(gc, go);
     if constexpr (kF64) {
@@ -207,7 +208,7 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
     }
     if (mode != 0) {
 #pragma unroll
-      for (int q = 0; q < kN; ++q) p[q] = ldcg(a.gg + c[q]);
+      for (int q = 0; q < kN; ++q) p[q] = a.gg[c[q]];
     }
 #pragma unroll
     for (int q = 0; q < kN; ++q) accumulate(A, d[q], go[q], mode != 0 ? project(p[q].x, p[q].y, alpha) : go[q]);
@@ -226,7 +227,7 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
       }
     }
   };
-  auto finish = [&](long long p, const CellAcc<Real>& A, const V4& cl, double uez) {
+  auto finish = [&](int p, const CellAcc<Real>& A, const V4& cl, double uez) {
     double ux, uy, wz;
     if constexpr (kF64) {
       ux = add(add(0.0, mul(cl.x, A.f0)), 0.0);
@@ -246,8 +247,8 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
       *eg = add(*eg, mul((double)cl.z, im));
     }
     if (final) {
-      double* Up = a.U + 6 * p;
-      double* Fp = a.F + 6 * p;
+      double* Up = a.U + 6 * (size_t)p;
+      double* Fp = a.F + 6 * (size_t)p;
       Up[0] = ux;
       Up[1] = uy;
       Up[2] = 0.0;
@@ -276,47 +277,47 @@ __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double
   // round ahead of their use.  Which warp does a cell changes nothing in its
   // sums.
   constexpr bool kDyn = !kTr && U::kGrid;
-  const long long W = U::warps(), units = (a.n + kCellsPerWarp - 1) / kCellsPerWarp;
-  const int grp = (int)(U::warp() % kTakeGroups);
+  const int W = (int)U::warps(), units = (int)((a.n + kCellsPerWarp - 1) / kCellsPerWarp), n = (int)a.n;
+  const int grp = (int)U::warp() % kTakeGroups;
   unsigned long long* take = kDyn ? &a.sc->take[set][grp][0] : nullptr;
-  long long ucur = U::warp(), unext = ucur + W;
-  long long p = ucur * kCellsPerWarp + lane / kLanes;
+  int ucur = (int)U::warp(), unext = ucur + W;
+  int p = ucur * kCellsPerWarp + lane / kLanes;
   int b = 0, e = 0;
   V4 cl{};
   double uez = 0.0;
   if constexpr (kDyn) {
     unext = units;
-    if (ucur < units && lane == 0) unext = W + grp + kTakeGroups * (long long)atomicAdd(take, 1ULL);
+    if (ucur < units && lane == 0) unext = W + grp + kTakeGroups * (int)atomicAdd(take, 1ULL);
   }
-  if (p < a.n) {
+  if (p < n) {
     b = a.inc_off[p];
     e = a.inc_off[p + 1];
     cl = a.cell[p];
-    if (a.uext) uez = a.uext[3 * p + 2];
+    if (a.uext) uez = a.uext[3 * (size_t)p + 2];
   }
   if constexpr (kDyn) unext = __shfl_sync(kFull, unext, 0);
   while (ucur < units) {
-    long long uafter = unext + W;
+    int uafter = unext + W;
     if constexpr (kDyn) {
       uafter = units;
-      if (unext < units && lane == 0) uafter = W + grp + kTakeGroups * (long long)atomicAdd(take, 1ULL);
+      if (unext < units && lane == 0) uafter = W + grp + kTakeGroups * (int)atomicAdd(take, 1ULL);
     }
-    const long long pn = unext * kCellsPerWarp + lane / kLanes;
+    const int pn = unext * kCellsPerWarp + lane / kLanes;
     int bn = 0, en = 0;
     V4 cln{};
     double uezn = 0.0;
-    if (pn < a.n) {
+    if (pn < n) {
       bn = a.inc_off[pn];
       en = a.inc_off[pn + 1];
       cln = a.cell[pn];
-      if (a.uext) uezn = a.uext[3 * pn + 2];
+      if (a.uext) uezn = a.uext[3 * (size_t)pn + 2];
     }
     CellAcc<Real> A;
     int k = b + gl;
     for (; k + (kAhead - 1) * kLanes < e; k += kAhead * kLanes) take_entries(A, k, Count<kAhead>());
     for (; k < e; k += kLanes) take_entries(A, k, Count<1>());
     combine(A);
-    if (gl == 0 && p < a.n) finish(p, A, cl, uez);
+    if (gl == 0 && p < n) finish(p, A, cl, uez);
     if constexpr (kDyn) uafter = __shfl_sync(kFull, uafter, 0);
     ucur = unext;
     unext = uafter;
@@ -340,13 +341,13 @@ __device__ __forceinline__ void reset_take(SolverScalars* sc, int set) {
 }
 
 template <class Real>
-__device__ __forceinline__ double planar_grad(const PArgs<Real>& a, long long c) {
+__device__ __forceinline__ double planar_grad(const PArgs<Real>& a, int c) {
   const int2 ij = a.ij[c];
   const auto n = a.nn[c];
   const auto t = a.tt[c];
   const auto s = a.ss[c];
-  const auto ui = ldcg256(a.u + ij.x);
-  const auto uj = ldcg256(a.u + ij.y);
+  const auto ui = ld256w(a.u + ij.x);
+  const auto uj = ld256w(a.u + ij.y);
   if constexpr (sizeof(Real) == 8) {
     double pd = 0.0;
     pd = add(pd, mul(n.x, ui.x));
@@ -371,19 +372,27 @@ __device__ __forceinline__ double planar_grad(const PArgs<Real>& a, long long c)
   }
 }
 
+// Constraints of chunk ch, and how many of a block's chunks have them kept in
+// shared memory (two 64-bit divisions otherwise).
+constexpr int kBounds = 8;
+__device__ __forceinline__ int2 chunk_range(int ch, long long m, long long nchunks) {
+  return make_int2((int)chunk_lo(ch, m, nchunks), (int)chunk_lo(ch + 1, m, nchunks));
+}
+
 // Constraint pass: new (gamma, g) over the constraint's pair and its two
 // incidence entries, chunk partials.  mode 0 evaluates g at gamma_0 (residual
 // only).
 template <class Real, class U, int kTr>
 __device__ __forceinline__ void constraint_pass(const PArgs<Real>& a, int mode, double alpha, bool check, double* sm,
-                                                double* smt) {
+                                                double* smt, const int2* bounds = nullptr) {
   double2* gg = a.gg;
-  for (long long ch = U::unit(); ch < a.nchunks; ch += U::units()) {
+  for (int ch = (int)U::unit(), round = 0; ch < (int)a.nchunks; ch += (int)U::units(), ++round) {
     double v[4] = {0, 0, 0, 0};
     double lin = 0.0;
-    const long long hi = chunk_lo(ch + 1, a.m, a.nchunks);
+    const int2 range = bounds && round < kBounds ? bounds[round] : chunk_range(ch, a.m, a.nchunks);
+    const int hi = range.y;
 #pragma unroll 2
-    for (long long c = chunk_lo(ch, a.m, a.nchunks) + U::t(); c < hi; c += kBlock) {
+    for (int c = range.x + U::t(); c < hi; c += kBlock) {
       const double2 s = gg[c];
       const double gam = mode == 0 ? s.x : project(s.x, s.y, alpha);
       const double g = planar_grad(a, c);
@@ -443,6 +452,8 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
     // published between blocks.  Block 0 records the scalars for the host
     // and zeroes the cell-unit counters of the next iteration.
     __shared__ double s_v[4];
+    __shared__ int2 s_bounds[kBounds];
+    if (threadIdx.x < kBounds) s_bounds[threadIdx.x] = chunk_range(blockIdx.x + threadIdx.x * nb, a.m, a.nchunks);
     auto reduce_all = [&](double v[4]) {
       reduce_partials<GridUnits>(a.partials, a.nchunks, v, sm);
       if (threadIdx.x == 0) {
@@ -457,7 +468,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
     cell_pass<Real, GridUnits, 0>(a, 0, 0.0, false, nullptr, nullptr, 0);
     if (!bar.sync()) return;
     if (recorder) reset_take(sc, 1);
-    constraint_pass<Real, GridUnits, 0>(a, 0, 0.0, true, sm, nullptr);
+    constraint_pass<Real, GridUnits, 0>(a, 0, 0.0, true, sm, nullptr, s_bounds);
     if (!bar.sync()) return;
     double v[4];
     reduce_all(v);
@@ -474,7 +485,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
       cell_pass<Real, GridUnits, 0>(a, 1, alpha, check, nullptr, nullptr, (int)(it & 1));
       if (!bar.sync()) return;
       if (recorder) reset_take(sc, (int)((it + 1) & 1));
-      constraint_pass<Real, GridUnits, 0>(a, 1, alpha, check, sm, nullptr);
+      constraint_pass<Real, GridUnits, 0>(a, 1, alpha, check, sm, nullptr, s_bounds);
       if (!bar.sync()) return;
       reduce_all(v);
       if (check && v[3] <= a.tol) conv = true;

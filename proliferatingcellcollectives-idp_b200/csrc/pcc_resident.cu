@@ -706,14 +706,14 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
       if constexpr (kCluster) {
         *reinterpret_cast<int4*>(u + q) = *reinterpret_cast<const int4*>(us + (size_t)F::kU * p + q);
       } else if constexpr (kF64) {
-        const double4 w = ldcg256(reinterpret_cast<const double4*>(a.u) + ((size_t)F::kU * p + q) / 4);
+        const double4 w = ld256w(reinterpret_cast<const double4*>(a.u) + ((size_t)F::kU * p + q) / 4);
         u[q] = w.x;
         u[q + 1] = w.y;
         u[q + 2] = w.z;
         u[q + 3] = w.w;
       } else {
         *reinterpret_cast<int4*>(u + q) =
-            __ldcg(reinterpret_cast<const int4*>(reinterpret_cast<const Real*>(a.u) + (size_t)F::kU * p + q));
+            *(reinterpret_cast<const int4*>(reinterpret_cast<const Real*>(a.u) + (size_t)F::kU * p + q));
       }
     }
   };
@@ -866,9 +866,16 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
       if (q < values) {
         const double* part = a.partials + (size_t)q * nch;
         double r = 0.0;
-        for (int ch = 32 * (warp & 7) + lane; ch < nch; ch += kBlock) {
-          const double y = ldcg(part + ch);
-          r = q == 3 ? (r < y ? y : r) : add(r, y);
+        constexpr int kAtOnce = 3;
+#pragma unroll 1
+        for (int ch = 32 * (warp & 7) + lane; ch < nch; ch += kAtOnce * kBlock) {
+          double y[kAtOnce];
+#pragma unroll
+          for (int z = 0; z < kAtOnce; ++z) y[z] = ch + z * kBlock < nch ? ldcg(part + ch + z * kBlock) : 0.0;
+#pragma unroll
+          for (int z = 0; z < kAtOnce; ++z) {
+            if (ch + z * kBlock < nch) r = q == 3 ? (r < y[z] ? y[z] : r) : add(r, y[z]);
+          }
         }
         r = tree32(r, q == 3);
         if (lane == 0) s_grp[warp] = r;

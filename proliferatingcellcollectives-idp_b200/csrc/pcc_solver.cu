@@ -89,7 +89,7 @@ __device__ __forceinline__ void cell_pass(const SolverArgs& a, int mode, const d
       const long long c = ent >> 1;
       const int side = ent & 1;
       const double gold = a.gamma[c];
-      const double gc = mode == 0 ? gold : project(ldcg(gprev_gam + c), ldcg(gprev_g + c), alpha);
+      const double gc = mode == 0 ? gold : project(gprev_gam[c], gprev_g[c], alpha);
       const double diff = sub(gc, gold);
       double D[6];
       if (side == 0) {
@@ -152,33 +152,42 @@ __device__ __forceinline__ void cell_pass(const SolverArgs& a, int mode, const d
   }
 }
 
+// A velocity row, as three 16-byte loads that L1 keeps for the row's next
+// reader (see ld256 on why that is allowed).
+__device__ __forceinline__ void load6(const double* row, double u[6]) {
+#pragma unroll
+  for (int q = 0; q < 6; q += 2) *reinterpret_cast<double2*>(u + q) = *reinterpret_cast<const double2*>(row + q);
+}
+
 // Pass B value for constraint c: phi_next(gamma) given U and dldot.
 __device__ __forceinline__ double constraint_grad(const SolverArgs& a, long long c) {
   const int i = a.gi[c], j = a.gj[c];
-  const double* Ui = a.U + 6 * (long long)i;
-  const double* Uj = a.U + 6 * (long long)j;
+  double ui[6], uj[6];
+  load6(a.U + 6 * (long long)i, ui);
+  load6(a.U + 6 * (long long)j, uj);
+  const double li = a.dl[i], lj = a.dl[j];
   const double Di[6] = {a.nx[c], a.ny[c], a.nz[c], a.tix[c], a.tiy[c], a.tiz[c]};
   const double Dj[6] = {-a.nx[c], -a.ny[c], -a.nz[c], a.tjx[c], a.tjy[c], a.tjz[c]};
   double pd = 0.0;
   // MatMult row c: ascending columns; gi < gj for every emitted constraint
   if (i < j) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Di[q], ldcg(Ui + q)));
+    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Di[q], ui[q]));
 #pragma unroll
-    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Dj[q], ldcg(Uj + q)));
+    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Dj[q], uj[q]));
   } else {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Dj[q], ldcg(Uj + q)));
+    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Dj[q], uj[q]));
 #pragma unroll
-    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Di[q], ldcg(Ui + q)));
+    for (int q = 0; q < 6; ++q) pd = add(pd, mul(Di[q], ui[q]));
   }
   double gr = 0.0;
   if (i < j) {
-    gr = add(gr, mul(a.si[c], ldcg(a.dl + i)));
-    gr = add(gr, mul(a.sj[c], ldcg(a.dl + j)));
+    gr = add(gr, mul(a.si[c], li));
+    gr = add(gr, mul(a.sj[c], lj));
   } else {
-    gr = add(gr, mul(a.sj[c], ldcg(a.dl + j)));
-    gr = add(gr, mul(a.si[c], ldcg(a.dl + i)));
+    gr = add(gr, mul(a.sj[c], lj));
+    gr = add(gr, mul(a.si[c], li));
   }
   // VecMAXPY(phi_next, {dt, -dt}, {phidot, growth})
   return add(a.phi[c], add(mul(a.dt, pd), mul(-a.dt, gr)));
