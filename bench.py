@@ -475,8 +475,11 @@ def run_ours(args):
     if errors is not None:
         line["mixed_vs_fp64"] = errors
     if rank == 0 and world == 1 and not args.no_cpu:
-        ref = reference_step_model(cells, dt0, phases_step, iters_step)
-        line["cpu_baseline"] = {
+        try:
+            ref = reference_step_model(cells, dt0, phases_step, iters_step)
+        except FileNotFoundError:  # the reference's sources were not there to build
+            ref = None
+        line["cpu_baseline"] = {"unavailable": "the reference's build is missing"} if ref is None else {
             "value": ref["cell_steps_per_s"], "unit": UNIT, "cores": 1, "kind": "reference",
             "sample": f"the reference's solver call (release build, one thread) on the same R={meta['radius']:.0f} "
                       f"colony with BBPGD capped at {REF_SAMPLE_ITERS[0]} and {REF_SAMPLE_ITERS[1]} iterations "
