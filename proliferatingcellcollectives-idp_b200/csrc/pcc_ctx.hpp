@@ -153,10 +153,7 @@ struct pcc_ctx {
   double sim_time = 0, radius = 0;
   long long launches = 0;
   int coop_blocks = 0;         // co-resident blocks of the general solver kernel
-  int coop_blocks_planar = 0;  // ... of the planar one
-  int coop_blocks_mixed = 0;   // ... of its mixed-precision form
-  int coop_planar_tr = 0;      // ... and of their traced forms
-  int coop_mixed_tr = 0;
+  int coop_planar[2][3] = {};  // ... of the planar ones: [mixed, FP64][traced, three blocks per SM, four]
 
   // VTK output: device snapshot, side stream and background writer
   pcc::DevBuf<double> vtk_dev;

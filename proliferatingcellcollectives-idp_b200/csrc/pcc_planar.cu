@@ -56,23 +56,22 @@ namespace pcc {
 
 namespace {
 
-// Entries of a lane whose loads are in flight together in the cell pass, and
-// co-resident blocks per SM of the multi-block form: with four entries ahead
-// three blocks fit the registers (a few spilled bytes cost a quarter: loop
-// counters are 32-bit).  Measured before the 32-byte and L1-resident row loads
-// (19.9 / 16.3 / 106 / 86 now), us per iteration, 44,700 cells
-// FP64 / mixed and 302,172 cells FP64 / mixed: one ahead, four blocks 24.0 / - /
-// - / 93.2; two, four 26.2 / 18.7 / 145.8 / 89.5; four, three 22.7 / 17.7 /
-// 110.8 / 91.1; four, two 21.4 / 17.8 / 114.8 / 100.5.
-constexpr int kAhead = 4;
-// ... and the chunk target, per operand precision.
-template <class Real>
-struct Occupancy {
-  static constexpr int kBlocksPerSm = 3;
-  static constexpr long long kChunks = kChunkTarget;
-};
-// the general (FP64) kernel cuts its chunks with the default target
-static_assert(Occupancy<double>::kChunks == kChunkTarget, "FP64 chunks must match the general kernel's");
+// The untraced kernel has two forms, by the blocks per SM that share the
+// registers: three blocks with four entries of a lane in flight in the cell
+// pass, and four blocks with two.  The first is the faster one per pass; the
+// second takes the sets of exactly kChunkTarget long chunks, which its 592
+// blocks reduce in one round, where 444 blocks need two, the second round with
+// one block on each SM.  Measured, us per iteration of whole ReLCP calls, three
+// blocks / four (the constraints are those of the last phase): FP64 466,000
+// 16.3 / 18.9, 723,000 19.7 / 21.5, 958,000 29.3 / 26.6, 1,224,000 36.2 / 29.3,
+// 1,844,000 49.4 / 49.0, 2,868,000 72.9 / 79.6; mixed 14.7 / 16.3, 16.0 / 16.8,
+// 21.1 / 19.5, 29.4 / 23.7, 38.7 / 36.6, 53.6 / 55.1.
+// Spilled registers cost more than either choice gives (loop counters are
+// 32-bit).  From 350,000 constraints on instead of 500,000 calls that end with
+// 466,000 to 848,000 take 1-4 % longer, from 650,000 on those that end with
+// 958,000 to 1,224,000 3-13 %.
+constexpr int kFewBlocks = 3, kManyBlocks = 4;
+constexpr long long kLongChunks = 500000;
 
 template <class Real>
 struct PT;
@@ -163,7 +162,7 @@ struct CellAcc {
 // takes one cell per round and loads the next cell's incidence range and
 // record while it walks the current cell's entries, so the two loads are in
 // flight together; each cell's sums do not depend on which group takes it.
-template <class Real, class U, int kTr>
+template <class Real, class U, int kTr, int kAhead>
 __device__ __forceinline__ void cell_pass(const PArgs<Real>& a, int mode, double alpha, bool final, double* eq,
                                           double* eg, int set = 0) {
   using V4 = typename PT<Real>::V4;
@@ -435,12 +434,11 @@ __device__ __forceinline__ void trace_cells(double* smt, double eq, double eg, d
   }
 }
 
-// Occupancy<Real>::kBlocksPerSm blocks per SM fit the register file, which
-// the chunk sizing (Occupancy<Real>::kChunks) assumes.
-template <class Real, int kTr>
-__global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerSm) k_bbpgd_planar(PArgs<Real> a) {
+template <class Real, int kTr, int kBlocks>
+__global__ void __launch_bounds__(kBlock, kTr ? 1 : kBlocks) k_bbpgd_planar(PArgs<Real> a) {
   __shared__ double sm[4 * (kBlock / 32)];
   __shared__ double smt[kTr ? 4 * kBlock : 1];
+  constexpr int kAhead = kBlocks == kManyBlocks ? 2 : 4;
   const int TR = kTr ? a.trace : 0;
   const unsigned nb = gridDim.x;
   SolverScalars* sc = a.sc;
@@ -465,7 +463,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
       for (int q = 0; q < 4; ++q) v[q] = s_v[q];
     };
     const bool recorder = blockIdx.x == 0 && threadIdx.x == 0;
-    cell_pass<Real, GridUnits, 0>(a, 0, 0.0, false, nullptr, nullptr, 0);
+    cell_pass<Real, GridUnits, 0, kAhead>(a, 0, 0.0, false, nullptr, nullptr, 0);
     if (!bar.sync()) return;
     if (recorder) reset_take(sc, 1);
     constraint_pass<Real, GridUnits, 0>(a, 0, 0.0, true, sm, nullptr, s_bounds);
@@ -482,7 +480,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
     bool conv = false;
     while (it < a.max_it) {
       const bool check = (it % 10) == 0;
-      cell_pass<Real, GridUnits, 0>(a, 1, alpha, check, nullptr, nullptr, (int)(it & 1));
+      cell_pass<Real, GridUnits, 0, kAhead>(a, 1, alpha, check, nullptr, nullptr, (int)(it & 1));
       if (!bar.sync()) return;
       if (recorder) reset_take(sc, (int)((it + 1) & 1));
       constraint_pass<Real, GridUnits, 0>(a, 1, alpha, check, sm, nullptr, s_bounds);
@@ -515,7 +513,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
   // gradient at gamma_0 and the initial residual (BBPGD.cpp:40-44)
   {
     double eq = 0.0, eg = 0.0;
-    cell_pass<Real, GridUnits, kTr>(a, 0, 0.0, false, &eq, &eg);
+    cell_pass<Real, GridUnits, kTr, kAhead>(a, 0, 0.0, false, &eq, &eg);
     if (TR) trace_cells(smt, eq, eg, a.tr_part);
   }
   if (!bar.sync()) return;
@@ -542,7 +540,7 @@ __global__ void __launch_bounds__(kBlock, kTr ? 1 : Occupancy<Real>::kBlocksPerS
     const bool check = (it % 10) == 0 || TR;
     {
       double eq = 0.0, eg = 0.0;
-      cell_pass<Real, GridUnits, kTr>(a, 1, alpha, check, &eq, &eg);
+      cell_pass<Real, GridUnits, kTr, kAhead>(a, 1, alpha, check, &eq, &eg);
       if (TR) trace_cells(smt, eq, eg, a.tr_part);
     }
     if (!bar.sync()) return;
@@ -663,7 +661,7 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
       (e = B::inc(ctx).reserve(ne + 1, 0, s)) || (e = B::cell(ctx).reserve(nn, 0, s)) ||
       (e = B::u(ctx).reserve(nn, 0, s)))
     return e;
-  const long long nchunks = chunk_count((long long)m, Occupancy<Real>::kChunks);
+  const long long nchunks = chunk_count((long long)m);
   if ((e = ctx->partials.reserve(4 * (nchunks + 1), 0, s))) return e;
   ConsView cv = ctx->cons.view();
   if (m) {
@@ -716,13 +714,15 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
   a.trace_cap = tr.trace_cap;
   void* args[] = {&a};
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], s);
-  const void* kern = tr.trace ? (const void*)k_bbpgd_planar<Real, 1> : (const void*)k_bbpgd_planar<Real, 0>;
-  int& coop = tr.trace ? (sizeof(Real) == 8 ? ctx->coop_planar_tr : ctx->coop_mixed_tr)
-                       : (sizeof(Real) == 8 ? ctx->coop_blocks_planar : ctx->coop_blocks_mixed);
+  const bool many = !tr.trace && nchunks == kChunkTarget && (long long)m >= kLongChunks;
+  const void* kern = tr.trace ? (const void*)k_bbpgd_planar<Real, 1, kFewBlocks>
+                     : many   ? (const void*)k_bbpgd_planar<Real, 0, kManyBlocks>
+                              : (const void*)k_bbpgd_planar<Real, 0, kFewBlocks>;
+  int& coop = ctx->coop_planar[sizeof(Real) == 8][tr.trace ? 0 : many ? 2 : 1];
   if (coop == 0) {
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0))) return e;
-    const int cap = Occupancy<Real>::kBlocksPerSm;
+    const int cap = many ? kManyBlocks : kFewBlocks;
     coop = (per_sm < cap ? per_sm : cap) * ctx->num_sms;
   }
   long long want = (long long)grid_for((long long)n * kLanes);
@@ -736,11 +736,7 @@ cudaError_t launch(pcc_ctx* ctx, double dt, const PlanarTrace& tr, int* kind) {
 
 }  // namespace
 
-long long planar_chunks(size_t m) {  // the larger of the two precisions' counts
-  const long long a = chunk_count((long long)m, Occupancy<double>::kChunks);
-  const long long b = chunk_count((long long)m, Occupancy<float>::kChunks);
-  return a > b ? a : b;
-}
+long long planar_chunks(size_t m) { return chunk_count((long long)m); }
 
 cudaError_t planar_bbpgd(pcc_ctx* ctx, double dt, bool mixed, const PlanarTrace& tr, int* kind) {
   return mixed ? launch<float>(ctx, dt, tr, kind) : launch<double>(ctx, dt, tr, kind);

@@ -54,6 +54,17 @@ def test_on_chip_solve_bit_identical_to_streaming(radius, over, tmp_path):
     assert_same(solve(cells, tmp_path, 0, **over), solve(cells, tmp_path, 2, **over))
 
 
+@pytest.mark.parametrize("radius", [120.0, 160.0])
+@pytest.mark.parametrize("over", FORMS[:2], ids=["fp64", "mixed"])
+def test_streaming_with_long_chunks_bit_identical_to_traced(over, radius, tmp_path):
+    """Phases on both sides of 500,000 constraints, where the untraced
+    streaming kernel changes from three to four blocks per SM."""
+    cells = squeezed(radius, 0.985)
+    a, b = solve(cells, tmp_path, 0, **over), solve(cells, tmp_path, 2, **over)
+    assert 500_000 < a[0]["n_constraints"] < 1_212_416  # 592 chunks of up to 2,048
+    assert_same(a, b)
+
+
 @pytest.mark.parametrize("over", FORMS, ids=["fp64", "mixed", "3d"])
 def test_one_cell_and_no_constraints(over, tmp_path):
     cells = {k: np.asarray(v, np.int32 if k == "age" else float) for k, v in abi.seed_cell(4).items()}
