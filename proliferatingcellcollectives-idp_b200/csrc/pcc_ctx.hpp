@@ -154,6 +154,7 @@ struct pcc_ctx {
   long long launches = 0;
   int coop_blocks = 0;         // co-resident blocks of the general solver kernel
   int coop_planar[2][3] = {};  // ... of the planar ones: [mixed, FP64][traced, three blocks per SM, four]
+  int cluster_most[3] = {-1, -1, -1};  // largest cluster of the on-chip solver's [mixed, FP64, 3D] form; -1: not asked yet
 
   // VTK output: device snapshot, side stream and background writer
   pcc::DevBuf<double> vtk_dev;

@@ -36,7 +36,6 @@
 //
 // k3D: six D components (colonies out of the plane, FP64 only); otherwise
 // the planar form's three, in FP64 or with FP32 operands (Real = float).
-#include <atomic>
 #include <cfloat>
 #include <cmath>
 
@@ -1009,13 +1008,11 @@ bool shape_for(long long m, long long n, long long nchunks, int phases, int nb, 
 }
 
 // Opts both forms into their shared memory and asks for the largest cluster
-// that a device can hold, once per device and kernel (a property of the device;
-// two threads that ask at once store the same answer).
+// that the device can hold (0: none), once per context and kernel: the opt-in
+// belongs to the CUDA context, which a program may reset between colonies.
 template <class Real, bool k3D>
-cudaError_t largest_cluster(int device, int* out) {
-  constexpr int kDevices = 64;
-  static std::atomic<int> known[kDevices];
-  if (device >= 0 && device < kDevices && (*out = known[device].load())) return cudaSuccess;
+cudaError_t largest_cluster(int* known) {
+  if (*known >= 0) return cudaSuccess;
   const void* kc = (const void*)k_bbpgd_res<Real, k3D, true>;
   const void* kg = (const void*)k_bbpgd_res<Real, k3D, false>;
   cudaError_t e;
@@ -1023,22 +1020,22 @@ cudaError_t largest_cluster(int device, int* out) {
       (e = cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost)) ||
       (e = cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
     return e;
-  cudaLaunchConfig_t q = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim = {kMaxCluster, 1, 1};
-  q.gridDim = dim3(kMaxCluster);
-  q.blockDim = dim3(kClusterThreads);
-  q.dynamicSmemBytes = kSmemMost;
-  q.attrs = at;
-  q.numAttrs = 1;
-  int fit = 0;
-  if (cudaOccupancyMaxActiveClusters(&fit, kc, &q) != cudaSuccess) {
+  int most = kMaxCluster;
+  for (; most > 0; most /= 2) {
+    cudaLaunchConfig_t q = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)most, 1, 1};
+    q.gridDim = dim3((unsigned)most);
+    q.blockDim = dim3(kClusterThreads);
+    q.dynamicSmemBytes = kSmemMost;
+    q.attrs = at;
+    q.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kc, &q) == cudaSuccess && fit > 0) break;
     cudaGetLastError();
-    fit = 0;
   }
-  *out = fit > 0 ? kMaxCluster : kMaxCluster / 2;
-  if (device >= 0 && device < kDevices) known[device].store(*out);
+  *known = most;
   return cudaSuccess;
 }
 
@@ -1051,8 +1048,8 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
   const void* kg = (const void*)k_bbpgd_res<Real, k3D, false>;
   cudaError_t e;
   *taken = false;
-  int cluster_max = 0;
-  if ((e = largest_cluster<Real, k3D>(ctx->device, &cluster_max))) return e;
+  int& cluster_max = ctx->cluster_most[k3D ? 2 : sizeof(Real) == 8];
+  if ((e = largest_cluster<Real, k3D>(&cluster_max))) return e;
   Shape sh;
   bool cluster = false;
   if (nchunks <= kClusterChunks) {
