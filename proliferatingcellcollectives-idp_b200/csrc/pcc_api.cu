@@ -286,36 +286,40 @@ pcc_status solve(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* out, bool en
   return rc;
 }
 
+// Every exit waits for the stream: no copy into the caller's arrays outlives
+// the call, whatever failed.
 pcc_status download_contacts(pcc_ctx* ctx, size_t m, pcc_contacts* o) {
   cudaStream_t s = ctx->stream;
-  auto cp_d = [&](double* dst, const double* src, size_t count) {
-    if (dst && count) cudaMemcpyAsync(dst, src, count * sizeof(double), cudaMemcpyDeviceToHost, s);
-  };
-  auto cp_i = [&](int* dst, const int* src) {
-    if (dst && m) cudaMemcpyAsync(dst, src, m * sizeof(int), cudaMemcpyDeviceToHost, s);
+  cudaError_t e = cudaSuccess;
+  auto copy = [&](void* dst, const void* src, size_t bytes) {
+    if (!e && dst && bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
   };
   ConsView v = ctx->cons.view();
-  cp_i(o->gid_i, v.gi);
-  cp_i(o->gid_j, v.gj);
-  cp_i(o->phase, v.phase);
-  cp_d(o->sd, v.sd, m);
-  cp_d(o->stress_i, v.si, m);
-  cp_d(o->stress_j, v.sj, m);
-  cp_d(o->gamma, v.gamma, m);
+  copy(o->gid_i, v.gi, m * sizeof(int));
+  copy(o->gid_j, v.gj, m * sizeof(int));
+  copy(o->phase, v.phase, m * sizeof(int));
+  copy(o->sd, v.sd, m * sizeof(double));
+  copy(o->stress_i, v.si, m * sizeof(double));
+  copy(o->stress_j, v.sj, m * sizeof(double));
+  copy(o->gamma, v.gamma, m * sizeof(double));
   // vectors are interleaved on the device and land in the caller's arrays as
   // they are (a host loop over 723,024 contacts took about as long as their
-  // transfer); one scratch serves the four in stream order
+  // transfer), in pieces through the packed records of the detection that
+  // found the contacts: the next detection writes those anew, so the download
+  // needs no memory of its own
   const double* trip[4][3] = {{v.nx, v.ny, v.nz}, {v.rix, v.riy, v.riz}, {v.rjx, v.rjy, v.rjz}, {v.cpx, v.cpy, v.cpz}};
   double* outs[4] = {o->normal, o->r_i, o->r_j, o->contact_point};
-  if (m && (outs[0] || outs[1] || outs[2] || outs[3])) {
-    CU(ctx->interleaved.reserve(3 * m, 0, s), "download contacts");
-    for (int f = 0; f < 4; ++f) {
-      if (!outs[f]) continue;
-      CU(interleave3(ctx, trip[f][0], trip[f][1], trip[f][2], m), "download contacts");
-      cp_d(outs[f], ctx->interleaved.p, 3 * m);
+  const size_t piece = ctx->pk.cap / 3;
+  for (int f = 0; f < 4; ++f) {
+    if (!outs[f]) continue;
+    for (size_t k = 0; !e && k < m; k += piece) {
+      const size_t count = m - k < piece ? m - k : piece;
+      e = interleave3(ctx, trip[f][0] + k, trip[f][1] + k, trip[f][2] + k, count, ctx->pk.p);
+      copy(outs[f] + 3 * k, ctx->pk.p, 3 * count * sizeof(double));
     }
   }
-  CU(cudaStreamSynchronize(s), "download contacts");
+  const cudaError_t done = cudaStreamSynchronize(s);
+  CU(e ? e : done, "download contacts");
   return PCC_OK;
 }
 

@@ -746,8 +746,8 @@ __global__ void k_interleave3(const double* __restrict__ x, const double* __rest
 
 }  // namespace
 
-cudaError_t interleave3(pcc_ctx* ctx, const double* x, const double* y, const double* z, size_t n) {
-  k_interleave3<<<grid_for((long long)(3 * n)), kBlock, 0, ctx->stream>>>(x, y, z, n, ctx->interleaved.p);
+cudaError_t interleave3(pcc_ctx* ctx, const double* x, const double* y, const double* z, size_t n, double* out) {
+  k_interleave3<<<grid_for((long long)(3 * n)), kBlock, 0, ctx->stream>>>(x, y, z, n, out);
   ctx->launches++;
   return cudaGetLastError();
 }

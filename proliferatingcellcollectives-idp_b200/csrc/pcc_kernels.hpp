@@ -35,8 +35,8 @@ cudaError_t detect_contacts(pcc_ctx* ctx, double tol, int phase, bool reuse, siz
 cudaError_t build_incidence(pcc_ctx* ctx, bool order);
 cudaError_t order_incidence(pcc_ctx* ctx);
 
-// ctx->interleaved[3 k + d] = component d of vector k, for n vectors.
-cudaError_t interleave3(pcc_ctx* ctx, const double* x, const double* y, const double* z, size_t n);
+// out[3 k + d] = component d of vector k, for n vectors.
+cudaError_t interleave3(pcc_ctx* ctx, const double* x, const double* y, const double* z, size_t n, double* out);
 
 // ---- pcc_solver.cu
 // Draws the Brownian U_ext of every cell (temperature > 0) from the context's
