@@ -150,7 +150,7 @@ struct pcc_ctx {
   long long iter = 0;
   double sim_time = 0, radius = 0;
   long long launches = 0;
-  int coop_blocks = 0;         // co-resident blocks of the general solver kernel
+  int coop_general[2] = {};    // co-resident blocks of the general solver kernel: [plain, traced]
   int coop_planar[2][3] = {};  // ... of the planar ones: [mixed, FP64][traced, three blocks per SM, four]
   int cluster_most[3] = {-1, -1, -1};  // largest cluster of the on-chip solver's [mixed, FP64, 3D] form; -1: not asked yet
 

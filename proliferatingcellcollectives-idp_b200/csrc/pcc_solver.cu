@@ -677,7 +677,7 @@ cudaError_t bbpgd_solve(pcc_ctx* ctx, double dt, long long* iterations, double* 
     a.trace_out = ctx->trace_dev.p;
     a.trace_cap = trace_cap;
     const void* kern = tracing ? (const void*)k_bbpgd<1> : (const void*)k_bbpgd<0>;
-    int& coop = ctx->coop_blocks;
+    int& coop = ctx->coop_general[tracing];
     if (coop == 0) {
       int per_sm = 0;
       if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0))) return e;

@@ -28,3 +28,7 @@ def run(name: str, tmp_path, *args, stdin: str | None = None) -> str:
 
 def test_contact_download_leaves_no_copy_in_flight(tmp_path):
     assert run("contact_download", tmp_path).startswith("ok")
+
+
+def test_general_solver_grids_fit_each_kernel(tmp_path):
+    assert run("solver_grids", tmp_path).startswith("ok")
