@@ -395,6 +395,7 @@ pcc_status pcc_destroy(pcc_ctx* ctx) {
     cudaStreamDestroy(ctx->vtk_stream);
   }
   if (ctx->vtk_ev) cudaEventDestroy(ctx->vtk_ev);
+  if (ctx->x_ev) cudaEventDestroy(ctx->x_ev);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (auto& e : ctx->ev)
     if (e) cudaEventDestroy(e);
@@ -470,6 +471,7 @@ pcc_status pcc_upload_cells(pcc_ctx* ctx, const pcc_cells* c, size_t n) {
   CU(colony_radius(ctx, &ctx->radius), "radius");
   ctx->box_known = true;
   ctx->flat = true;
+  ctx->x_crowded = -1;
   return PCC_OK;
 }
 

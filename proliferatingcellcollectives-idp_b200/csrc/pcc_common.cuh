@@ -61,7 +61,7 @@ struct DevStatus {
   unsigned long long radius_bits;  // colony radius
   unsigned long long median[2];    // the two middle adaptDt speeds, as ordered keys
   int divisions;                   // of the next step
-  int pad2;
+  int crowded;                     // the last x-sort by buckets met a crowded one
   SolverScalars solver;  // of the last BBPGD launch
 };
 // What the host reads, in one copy: everything but the cell-unit counters.

@@ -138,6 +138,8 @@ struct pcc_ctx {
   double bbpgd_pending_bytes = 0.0;         // its algorithmic bytes per iteration
   bool mobility_known = false;              // Mlin / Mrot describe the resident cells
   double solved_overlap = 0.0;              // largest overlap that the last solve left
+  int x_crowded = -1;                       // cells crowd buckets of the x-sort: 1, do not: 0, not seen since the upload: -1
+  cudaEvent_t x_ev = nullptr;               // the answer to that is on the host
   bool div_known = false;                   // div_flag / div_off / div_next describe the resident cells
   size_t div_next = 0;                      // divisions the next step commits
 

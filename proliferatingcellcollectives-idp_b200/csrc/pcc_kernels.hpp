@@ -10,6 +10,7 @@ namespace pcc {
 // Slots of ctx->pinned_ll for values copied back at a synchronisation point.
 constexpr int kSlotRadius = 10;  // colony radius bits
 constexpr int kSlotDivs = 11;    // divisions of the next step
+constexpr int kSlotCrowded = 12;  // a crowded bucket of the x-sort
 
 // ---- pcc_scan_sort.cu
 // out[i] = sum in[0..i-1] for i in [0, n]; out has n+1 entries.  The sum of

@@ -215,9 +215,16 @@ __global__ void __launch_bounds__(kBlock) k_rank_sort(CellsView src, CellsView d
 // The x-sort of a larger colony: two buckets per cell over [-r, r] in x (r the
 // colony radius; cells beyond it fall in the end buckets), then each cell's
 // rank among its bucket's cells by (key, index).  Buckets hold about half a
-// cell each; a bucket of k cells costs k comparisons for each of them, so a
-// colony standing in one column still sorts, in n^2 / (GPU width).  Five
-// launches where the radix sort of the 64-bit keys took 24.
+// cell each; five launches where a radix sort of the 64-bit keys takes 24.  A
+// bucket of k cells costs k comparisons for each of them, so a colony with
+// more than kBucketMost cells in one (a tall one whose cells share few x, one
+// stretched by a far outlier) takes the radix sort, whose cost does not depend
+// on the keys.  Steps of separate cells, buckets / radix, ms, by the cells in
+// each bucket: 17,000 cells, 4,000 0.46 / 0.28, 1,000 0.26 / 0.27; 300,000
+// cells, 300,000 69.0 / 0.50, 9,000 2.44 / 0.51, 1,000 0.60 / 0.52, 700
+// 0.53 / 0.52, 400 0.45 / 0.52; 1,000,000 cells, 2,000 2.23 / 1.07, 700
+// 1.31 / 1.06, 400 1.09 / 1.06.
+constexpr int kBucketMost = 256;
 struct Buckets {
   double lo, scale;
   int count;
@@ -229,21 +236,27 @@ struct Buckets {
 };
 
 __global__ void k_bucket_count(const double* __restrict__ x, long long n, Buckets bk, int* __restrict__ cnt,
-                               int* __restrict__ arrival) {
+                               int* __restrict__ arrival, int* __restrict__ crowded) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) arrival[i] = atomicAdd(&cnt[bk.of(x[i])], 1);
+  if (i >= n) return;
+  const int at = atomicAdd(&cnt[bk.of(x[i])], 1);
+  arrival[i] = at;
+  if (at == kBucketMost) *crowded = 1;
 }
 
 __global__ void k_bucket_place(const double* __restrict__ x, long long n, Buckets bk, const int* __restrict__ off,
-                               const int* __restrict__ arrival, int* __restrict__ cells) {
+                               const int* __restrict__ arrival, const int* __restrict__ crowded,
+                               int* __restrict__ cells, DevStatus* st) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) st->crowded = *crowded;
   if (i < n) cells[off[bk.of(x[i])] + arrival[i]] = (int)i;
 }
 
+// skip: leave dst alone if the buckets are crowded (the host then sorts by radix); null: sort them all the same.
 __global__ void k_bucket_gather(CellsView src, CellsView dst, long long n, Buckets bk, const int* __restrict__ off,
-                                const int* __restrict__ cells) {
+                                const int* __restrict__ cells, const int* __restrict__ skip) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
+  if (s >= n || (skip && *skip)) return;
   const int i = cells[s];
   const double x = src.x[i];
   const unsigned long long mine = double_key(x);
@@ -255,6 +268,19 @@ __global__ void k_bucket_gather(CellsView src, CellsView dst, long long n, Bucke
     j += (key < mine || (key == mine && o < i)) ? 1 : 0;
   }
   move_cell(src, dst, i, j);
+}
+
+__global__ void k_x_keys(const double* __restrict__ x, long long n, unsigned long long* __restrict__ keys,
+                         int* __restrict__ perm) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  keys[i] = double_key(x[i]);
+  perm[i] = (int)i;
+}
+
+__global__ void k_gather_cells(CellsView src, CellsView dst, const int* __restrict__ perm, long long n) {
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) move_cell(src, dst, perm[j], j);
 }
 
 // Distance of a cell's far end from the origin (spatial/Domain.cpp:148-153).
@@ -399,16 +425,41 @@ cudaError_t sort_cells_by_x(pcc_ctx* ctx) {
     bk.lo = -r;
     bk.scale = bk.count / (2.0 * r);
     if ((e = ctx->perm.reserve(n, 0, s)) || (e = ctx->perm_alt.reserve(n, 0, s)) ||
-        (e = ctx->sort_hist.reserve(2 * (size_t)bk.count + 1, 0, s)))
+        (e = ctx->sort_hist.reserve(2 * (size_t)bk.count + 2, 0, s)))
       return e;
-    int *cnt = ctx->sort_hist.p, *off = cnt + bk.count;
-    cudaMemsetAsync(cnt, 0, bk.count * sizeof(int), s);
-    k_bucket_count<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, cnt, ctx->perm_alt.p);
-    if ((e = exclusive_scan(ctx, cnt, off, bk.count))) return e;
-    k_bucket_place<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, off, ctx->perm_alt.p, ctx->perm.p);
-    k_bucket_gather<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), (long long)n, bk, off,
-                                                  ctx->perm.p);
-    ctx->launches += 3;
+    int *cnt = ctx->sort_hist.p, *crowded = cnt + bk.count, *off = crowded + 1;
+    // the first such sort since the upload asks whether the buckets are crowded
+    // (the answer comes while the sort runs), a later one goes by the step before
+    const bool ask = ctx->x_crowded < 0;
+    int* flag = reinterpret_cast<int*>(ctx->pinned_ll + kSlotCrowded);
+    if (ctx->x_crowded <= 0) {
+      cudaMemsetAsync(cnt, 0, (bk.count + 1) * sizeof(int), s);
+      k_bucket_count<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, cnt, ctx->perm_alt.p, crowded);
+      if (ask) {
+        if (!ctx->x_ev && (e = cudaEventCreateWithFlags(&ctx->x_ev, cudaEventDisableTiming))) return e;
+        if ((e = cudaMemcpyAsync(flag, crowded, sizeof(int), cudaMemcpyDeviceToHost, s)) ||
+            (e = cudaEventRecord(ctx->x_ev, s)))
+          return e;
+      }
+      if ((e = exclusive_scan(ctx, cnt, off, bk.count))) return e;
+      k_bucket_place<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, bk, off, ctx->perm_alt.p, crowded,
+                                                    ctx->perm.p, ctx->status);
+      k_bucket_gather<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), (long long)n, bk, off,
+                                                    ctx->perm.p, ask ? crowded : nullptr);
+      ctx->launches += 3;
+    }
+    if (ask) {
+      if ((e = cudaEventSynchronize(ctx->x_ev))) return e;
+      ctx->x_crowded = *flag;
+    }
+    if (ctx->x_crowded > 0) {
+      if ((e = ctx->keys.reserve(n, 0, s))) return e;
+      k_x_keys<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.x.p, (long long)n, ctx->keys.p, ctx->perm.p);
+      if ((e = radix_sort_pairs(ctx, ctx->keys.p, ctx->perm.p, n, 64))) return e;
+      k_gather_cells<<<grid_for(n), kBlock, 0, s>>>(ctx->cells.view(), ctx->cells_alt.view(), ctx->perm.p,
+                                                    (long long)n);
+      ctx->launches += 2;
+    }
   }
   ctx->cells.swap(ctx->cells_alt);
   return cudaGetLastError();
@@ -486,6 +537,7 @@ void step_end_collect(pcc_ctx* ctx) {
   if (!ctx->params.fixed_dt) adapt_dt(ctx);
   std::memcpy(&ctx->radius, &st.radius_bits, sizeof ctx->radius);
   ctx->box_known = true;
+  if (ctx->x_crowded == 0) ctx->x_crowded = st.crowded;
   ctx->div_next = (size_t)st.divisions;
   ctx->div_known = true;
 }

@@ -45,3 +45,30 @@ def test_first_detection_of_a_solid_colony():
     r = N ** (1 / 3)
     first, later = first_and_later(rods(*rng.uniform(-r, r, (3, N)), rng))
     assert first < 8 * later, (first, later)
+
+
+@pytest.mark.parametrize("columns", [1, 32])
+def test_sort_of_a_tall_colony(columns):
+    """Its cells share few x."""
+    rng = np.random.default_rng(1)
+    k = np.arange(N)
+    square = int(np.sqrt(N))
+    usual = first_and_later(rods(4.0 * (k % square), 4.0 * (k // square), np.zeros(N), rng))
+    tall = first_and_later(rods(4.0 * (k % columns), 4.0 * (k // columns), np.zeros(N), rng))
+    assert tall[0] < 4 * usual[0] and tall[1] < 4 * usual[1], (tall, usual)
+
+
+def test_order_of_a_colony_that_crowds_and_spreads():
+    """The x-sort on both sides of its change of form, after one another on one context: the order is a stable sort."""
+    rng = np.random.default_rng(2)
+    n = 40_000
+    k = rng.permutation(n)
+    g = Colony(abi.default_params(mode=abi.MODE_SOFT, kcc=1000.0, dt=1e-7, fixed_dt=1, ghost_mode=abi.GHOSTS_NONE))
+    for columns in (400, 1, 156, 157, 400, 155):  # 100, 40,000, 257, 255, 100, 259 cells to a bucket
+        cells = rods(4.0 * (k % columns) - 2.0 * columns, 4.0 * (k // columns) + 0.5, np.zeros(n), rng)
+        g.set_cells(cells)
+        for _ in range(2):
+            g.step()
+            got, o = g.get_cells(), np.argsort(cells["x"], kind="stable")
+            np.testing.assert_array_equal(got["x"], cells["x"][o])
+            np.testing.assert_array_equal(got["y"], cells["y"][o])
