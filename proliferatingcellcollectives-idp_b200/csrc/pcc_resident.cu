@@ -28,7 +28,13 @@
 //     entry, so an iteration pays one gather latency.
 // A group of cells that does not fit the block's room (an unusually crowded
 // range) is read from the constraints themselves at every use; the host sizes
-// the room so that this does not happen in ordinary colonies.
+// the room so that this does not happen in ordinary colonies.  What bounds such
+// a group is the chain of its longest cell's entries, each a load of the entry
+// and then of its constraint: with the next entry's load in flight, 800 knotted
+// cells of up to 183 entries beside 28,000 sparse ones (59 groups without room,
+// FP64) take 68.6 -> 54.0 us per iteration (the streaming kernel's form of one
+// entry at a time took 57.6), 300 beside 2,000 (six, mixed, 16 blocks) 31.8 ->
+// 25.5 (29.4).
 //
 // Measured, us per iteration before (streaming kernels) and now, B200 at 1965
 // MHz: 447 cells / 3,000 constraints FP64 18.7 -> 4.3; 1,788 / 12,000 FP64 15.5
@@ -204,7 +210,7 @@ __device__ __forceinline__ double tree8(const double w[8], bool is_max) {
 
 // First cell whose weight (its offset in the incidence list + kappa per cell
 // before it) reaches block b's share.
-__device__ __forceinline__ int first_cell(const int* __restrict__ off, long long n, long long kappa, long long b,
+__host__ __device__ __forceinline__ int first_cell(const int* __restrict__ off, long long n, long long kappa, long long b,
                                           long long nb) {
   if (b >= nb) return (int)n;
   const long long total = (long long)off[n] + kappa * n, want = (b * total + nb - 1) / nb;
@@ -597,9 +603,12 @@ __global__ void __launch_bounds__(kCluster ? kClusterThreads : kGridThreads, 1) 
           take(r, p.x, p.y);
         }
       } else {  // no room in shared memory
+        const int* list = a.inc_ent + eb + soff[pl];
+        int next = l < d ? list[l] : 0;
 #pragma unroll 1
-        for (int k = soff[pl] + l; k < soff[pl] + d; k += kLanes) {
-          const int ent = a.inc_ent[eb + k];
+        for (int k = l; k < d; k += kLanes) {
+          const int ent = next;
+          if (k + kLanes < d) next = list[k + kLanes];  // in flight beside this entry's loads
           Real r[F::kRow];
           load_row(ent, r);
           const double go = a.cs.gamma[ent >> 1];
@@ -1007,6 +1016,23 @@ bool shape_for(long long m, long long n, long long nchunks, int phases, int nb, 
   return o->smem <= kSmemMost;
 }
 
+// The form and shape for m constraints, found in `phases` detections, on n
+// cells: the smallest cluster that leaves a block at most kClusterShare
+// constraints (or the largest, if its shared memory holds them), else the grid
+// form; false: neither holds them.
+template <class Real, bool k3D>
+bool pick_shape(long long m, long long n, int phases, int num_sms, int cluster_max, Shape* sh, bool* cluster) {
+  const long long nchunks = chunk_count(m);
+  *cluster = false;
+  if (nchunks <= kClusterChunks) {
+    for (int nb = 1; nb <= cluster_max && !*cluster; nb *= 2) {
+      if (nb < cluster_max && m > (long long)nb * kClusterShare) continue;
+      *cluster = shape_for<Real, k3D, true>(m, n, nchunks, phases, nb, sh);
+    }
+  }
+  return *cluster || shape_for<Real, k3D, false>(m, n, nchunks, 1, (int)(nchunks < num_sms ? nchunks : num_sms), sh);
+}
+
 // Opts both forms into their shared memory and asks for the largest cluster
 // that the device can hold (0: none), once per context and kernel: the opt-in
 // belongs to the CUDA context, which a program may reset between colonies.
@@ -1052,14 +1078,7 @@ cudaError_t try_resident(pcc_ctx* ctx, double dt, bool* taken, int* kind) {
   if ((e = largest_cluster<Real, k3D>(&cluster_max))) return e;
   Shape sh;
   bool cluster = false;
-  if (nchunks <= kClusterChunks) {
-    for (int nb = 1; nb <= cluster_max && !cluster; nb *= 2) {
-      if (nb < cluster_max && m > (long long)nb * kClusterShare) continue;
-      cluster = shape_for<Real, k3D, true>(m, n, nchunks, ctx->trace_phase + 1, nb, &sh);
-    }
-  }
-  const int blocks = (int)(nchunks < ctx->num_sms ? nchunks : ctx->num_sms);
-  if (!cluster && !shape_for<Real, k3D, false>(m, n, nchunks, 1, blocks, &sh)) return cudaSuccess;
+  if (!pick_shape<Real, k3D>(m, n, ctx->trace_phase + 1, ctx->num_sms, cluster_max, &sh, &cluster)) return cudaSuccess;
   if ((e = ctx->p_gg.reserve(m + 1, 0, s)) || (e = ctx->p_phin.reserve(m + 1, 0, s)) ||
       (e = ctx->partials.reserve(4 * (nchunks + 1), 0, s)) || (e = ctx->p_u.reserve(2 * (n + 1), 0, s)))
     return e;
