@@ -291,8 +291,16 @@ def start_state() -> tuple[dict, float, dict]:
 
 
 def run_reference(args):
-    world, rank = int(os.environ.get("WORLD_SIZE", "1")), int(os.environ.get("RANK", "0"))
+    rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    sys.path.insert(0, str(ROOT / "tests"))
+    from oracles import RefColony, ReferenceUnavailable
+    try:
+        RefColony(colony_params(), fast=True)
+    except ReferenceUnavailable:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's build is missing and its sources were "
+                                                              "not there to build it"}), flush=True)
         return
     cells, dt, meta = start_state()
     n = len(cells["x"])

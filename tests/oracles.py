@@ -22,10 +22,15 @@ REPO = Path(__file__).resolve().parents[1]
 REF_DIR = REPO / "oracle" / "_ref"
 
 
+class ReferenceUnavailable(FileNotFoundError):
+    """The reference's own build is not there."""
+
+
 def _load(name: str):
     path = REF_DIR / name
     if not path.exists():
-        raise FileNotFoundError(f"{path} is missing: run `make -C oracle` (or __graft_entry__.build())")
+        kind = ReferenceUnavailable if name.startswith("libpccref") else FileNotFoundError
+        raise kind(f"{path} is missing: run `make -C oracle` (or __graft_entry__.build())")
     return C.CDLL(str(path))
 
 
