@@ -159,7 +159,8 @@ typedef struct pcc_profile {
   long long bbpgd_launches;     /* persistent BBPGD kernel launches */
   long long bbpgd_iterations;   /* iterations they ran */
   double bbpgd_ms;              /* device time of those launches */
-  double bbpgd_algo_bytes;      /* sum over launches of iterations * (312 C + 288 N); (192 C + 144 N) mixed */
+  double bbpgd_algo_bytes;      /* sum over launches of iterations * (312 C + 288 N); (192 C + 144 N) mixed: every
+                                   operand at every use, whatever cache or shared memory it comes from */
   double detect_ms;             /* contact detection + incidence lists */
   double solve_ms;              /* whole pcc_solve calls */
   long long solves;
