@@ -22,12 +22,14 @@ constexpr int kTraceWidth = 8;  // it, residual, step size, linear, quadratic, g
 // taking the chunk's constraints lo + t, lo + t + 256, ... and summing its
 // terms in that order before the unit's fixed shuffle tree.  The count
 // depends on the constraint count alone: one constraint per thread while
-// that needs at most kChunkTarget chunks, else kChunkTarget chunks (one
-// round of a grid of four 256-thread blocks on each of 148 SMs, so every
-// block reduces one chunk per iteration), else as many as keep a thread at
-// kMaxPerThread constraints.  Nothing depends on the grid.
+// that needs at most kChunkTarget chunks, else kChunkTarget chunks, else as
+// many as keep a thread at kMaxPerThread constraints.  kChunkTarget is four
+// 256-thread blocks on each of 148 SMs: the streaming planar kernel's grid of
+// four blocks per SM reduces that many in one round, its three blocks per SM
+// (444) and the general kernel's two (296) in two.  Nothing depends on the
+// grid.
 constexpr int kLanes = 2;
-constexpr long long kChunkTarget = 592;  // 4 blocks on each of 148 SMs
+constexpr long long kChunkTarget = 592;
 constexpr int kMaxPerThread = 8;
 __host__ __device__ inline long long chunk_count(long long m, long long target = kChunkTarget) {
   long long c = (m + kBlock - 1) / kBlock;
@@ -241,8 +243,11 @@ __device__ __forceinline__ double bb_step(const double v[4], long long it) {
   return step > 0.0 ? step : 0.0;
 }
 
-// Work units.  A unit is 256 threads; chunk ch belongs to unit ch % units.
-struct GridUnits {  // the multi-block kernel: one unit per block
+// Work units of the streaming kernels, one 256-thread unit per block; chunk ch
+// belongs to unit ch % units.  A template argument of the passes though no
+// other kind is left: with the calls written out in their place ptxas spills
+// 24 and 32 bytes in the loops of the mixed kernels, and none with them.
+struct GridUnits {
   static constexpr bool kGrid = true;
   __device__ static unsigned units() { return gridDim.x; }
   __device__ static unsigned unit() { return blockIdx.x; }

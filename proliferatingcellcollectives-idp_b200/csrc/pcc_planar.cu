@@ -58,18 +58,26 @@ namespace {
 
 // The untraced kernel has two forms, by the blocks per SM that share the
 // registers: three blocks with four entries of a lane in flight in the cell
-// pass, and four blocks with two.  The first is the faster one per pass; the
-// second takes the sets of exactly kChunkTarget long chunks, which its 592
-// blocks reduce in one round, where 444 blocks need two, the second round with
-// one block on each SM.  Measured, us per iteration of whole ReLCP calls, three
-// blocks / four (the constraints are those of the last phase): FP64 466,000
-// 16.3 / 18.9, 723,000 19.7 / 21.5, 958,000 29.3 / 26.6, 1,224,000 36.2 / 29.3,
-// 1,844,000 49.4 / 49.0, 2,868,000 72.9 / 79.6; mixed 14.7 / 16.3, 16.0 / 16.8,
-// 21.1 / 19.5, 29.4 / 23.7, 38.7 / 36.6, 53.6 / 55.1.
-// Spilled registers cost more than either choice gives (loop counters are
-// 32-bit).  From 350,000 constraints on instead of 500,000 calls that end with
-// 466,000 to 848,000 take 1-4 % longer, from 650,000 on those that end with
-// 958,000 to 1,224,000 3-13 %.
+// pass, and four blocks with two.  The second takes sets of exactly
+// kChunkTarget long chunks, which its 592 blocks reduce in one round, where 444
+// blocks need two, the second round with one block on each SM.  Measured, us
+// per iteration, three blocks / four, on the constraints of one detection of a
+// dense packing: FP64 170,516 14.7 / 13.6, 207,223 15.6 / 15.2, 291,819 18.7 /
+// 18.3, 360,205 21.4 / 21.5, 456,347 26.0 / 26.9, 519,809 31.7 / 30.6, 654,571
+// 38.4 / 36.8, 1,101,179 57.0 / 54.5; mixed 13.1 / 11.5, 14.2 / 12.3, 16.0 /
+// 15.3, 17.3 / 16.0, 19.4 / 17.6, 22.0 / 18.7, 25.6 / 21.7, 41.9 / 38.1.  Over
+// whole ReLCP calls, whose later phases repeat pairs (named by the last phase's
+// constraints; the earlier ones are smaller): FP64 466,000 16.3 / 18.9, 723,000
+// 19.7 / 21.5, 958,000 29.3 / 26.6, 1,224,000 36.2 / 29.3, 1,844,000 49.4 /
+// 49.0, 2,868,000 72.9 / 79.6; mixed 14.7 / 16.3, 16.0 / 16.8, 21.1 / 19.5,
+// 29.4 / 23.7, 38.7 / 36.6, 53.6 / 55.1.  A step's phases start with one
+// detection's set and grow from it, so the line lies between the two: from
+// 350,000 constraints on instead, calls that end with 466,000 to 848,000 take
+// 1-4 % longer, from 650,000 on those that end with 958,000 to 1,224,000
+// 3-13 %.  Registers spilled within the loops cost more than either choice
+// gives (their counters are 32-bit for that); what is left, 16 bytes stored with
+// three blocks in FP64 and 116 with four, none in mixed precision, is in these
+// figures.
 constexpr int kFewBlocks = 3, kManyBlocks = 4;
 constexpr long long kLongChunks = 500000;
 
@@ -378,9 +386,8 @@ __device__ __forceinline__ int2 chunk_range(int ch, long long m, long long nchun
   return make_int2((int)chunk_lo(ch, m, nchunks), (int)chunk_lo(ch + 1, m, nchunks));
 }
 
-// Constraint pass: new (gamma, g) over the constraint's pair and its two
-// incidence entries, chunk partials.  mode 0 evaluates g at gamma_0 (residual
-// only).
+// Constraint pass: new (gamma, g) over the constraint's pair, chunk partials.
+// mode 0 evaluates g at gamma_0 (residual only).
 template <class Real, class U, int kTr>
 __device__ __forceinline__ void constraint_pass(const PArgs<Real>& a, int mode, double alpha, bool check, double* sm,
                                                 double* smt, const int2* bounds = nullptr) {
