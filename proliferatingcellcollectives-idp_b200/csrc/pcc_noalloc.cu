@@ -25,16 +25,14 @@
 // GPU (two streams, or two host threads) race on the scratch and must not be
 // issued concurrently on one device.
 //
-// The first call on each device resolves the device address of the scratch
-// array with cudaGetSymbolAddress while that device is current (the host-side
-// name of a __device__ array is only a stand-in and must never be passed to a
-// kernel); later calls reuse the cached address.  Make the first call on a
-// device before any stream capture on it.  With lazy module loading (the
-// CUDA 12 default) that first call, and the first launch of each kernel here,
-// may also make the driver load this file's device code, which takes device
-// memory of the driver's own; warm calls allocate nothing.
+// Every call resolves the device address of the scratch array with
+// cudaGetSymbolAddress while its device is current (the host-side name of a
+// __device__ array is only a stand-in and must never be passed to a kernel).
+// With lazy module loading (the CUDA 12 default) the first call on a device,
+// and the first launch of each kernel here, may also make the driver load this
+// file's device code, which takes device memory of the driver's own; warm calls
+// allocate nothing.
 #include <cstdio>
-#include <mutex>
 
 #include "pcc_common.cuh"
 
@@ -42,7 +40,6 @@ namespace {
 
 constexpr long long kNoallocMaxCells = 65536;
 constexpr long long kNoallocMaxContacts = 393216;
-constexpr int kNoallocMaxDevices = 64;
 
 // Scratch layout (bytes, each part 256-byte aligned):
 //   fel       kNoallocMaxContacts doubles     Hertz force magnitudes
@@ -59,9 +56,6 @@ constexpr size_t kFlagBytes = 256;
 constexpr size_t kScratchBytes = kFelBytes + 3 * kCellIntBytes + kEntBytes + kFlagBytes;  // 6.75 MiB
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
-
-std::mutex g_noalloc_mu;
-void* g_noalloc_ptr[kNoallocMaxDevices] = {};
 
 __device__ __forceinline__ double pow15_na(double x) {
   const double s = __dsqrt_rn(x);
@@ -269,21 +263,13 @@ extern "C" pcc_status pcc_soft_forces_noalloc(const int* gid_i, const int* gid_j
   // an error left pending by earlier work in the process is not this call's:
   // report it without launching (and without clearing it)
   if (cudaPeekAtLastError() != cudaSuccess) return PCC_ERR_CUDA;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNoallocMaxDevices) return PCC_ERR_CUDA;
+  // asked at every call: the array belongs to the current CUDA context, which
+  // the program may reset between calls
   void* base = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    if (!g_noalloc_ptr[dev]) {
-      void* p = nullptr;
-      cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-      if (e != cudaSuccess || !p) {
-        std::fprintf(stderr, "pcc_soft_forces_noalloc: cudaGetSymbolAddress failed: %s\n", cudaGetErrorString(e));
-        return PCC_ERR_CUDA;
-      }
-      g_noalloc_ptr[dev] = p;
-    }
-    base = g_noalloc_ptr[dev];
+  const cudaError_t e = cudaGetSymbolAddress(&base, g_noalloc_scratch);
+  if (e != cudaSuccess || !base) {
+    std::fprintf(stderr, "pcc_soft_forces_noalloc: cudaGetSymbolAddress failed: %s\n", cudaGetErrorString(e));
+    return PCC_ERR_CUDA;
   }
   unsigned char* b = static_cast<unsigned char*>(base);
   double* fel = reinterpret_cast<double*>(b);

@@ -90,3 +90,7 @@ def test_on_chip_solver_takes_the_forms_its_tests_name(tmp_path):
     for got, expect in zip(out, want):
         form, _, without = got.split()
         assert expect is None or (form, int(without)) == expect, (got, expect)
+
+
+def test_noalloc_scratch_is_the_current_contexts(tmp_path):
+    assert run("noalloc_scratch", tmp_path).startswith("ok")
