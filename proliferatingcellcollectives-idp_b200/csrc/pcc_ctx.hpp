@@ -91,7 +91,7 @@ struct pcc_ctx {
   pcc::DevBuf<int> ghost;
   bool box_known = false;  // radius bounds the centres of the resident cells
   bool flat = true;        // no cell left the plane z = 0 since the upload
-  // candidate partner lists of the last full neighbourhood pass (list-major)
+  // candidate partner lists of the last full neighbourhood pass (a cell's slots together)
   pcc::DevBuf<int> plist, plist_n, slot_of;
   pcc::DevBuf<double> xref;  // cell positions when the lists were built
   bool list_valid = false;
