@@ -290,6 +290,25 @@ pcc_status solve(pcc_ctx* ctx, double dt, int iter, pcc_step_stats* out, bool en
 // the call, whatever failed.
 pcc_status download_contacts(pcc_ctx* ctx, size_t m, pcc_contacts* o) {
   cudaStream_t s = ctx->stream;
+  // vectors are interleaved on the device and land in the caller's arrays as
+  // they are (a host loop over 723,024 contacts took about as long as their
+  // transfer).  One scratch serves the four in stream order; a device too full
+  // for it interleaves in pieces through the packed records of the detection
+  // that found the contacts, which the next detection writes anew (pieces for
+  // all: 852 us for a call on a small colony that takes 793)
+  double* scratch = ctx->pk.p;
+  size_t piece = ctx->pk.cap / 3;
+  if (m && (o->normal || o->r_i || o->r_j || o->contact_point)) {
+    const cudaError_t full = ctx->interleaved.reserve(3 * m, 0, s);
+    if (!full) {
+      scratch = ctx->interleaved.p;
+      piece = m;
+    } else if (full == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // handled
+    } else {
+      return cuda_fail(ctx, full, "download contacts");
+    }
+  }
   cudaError_t e = cudaSuccess;
   auto copy = [&](void* dst, const void* src, size_t bytes) {
     if (!e && dst && bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
@@ -302,20 +321,14 @@ pcc_status download_contacts(pcc_ctx* ctx, size_t m, pcc_contacts* o) {
   copy(o->stress_i, v.si, m * sizeof(double));
   copy(o->stress_j, v.sj, m * sizeof(double));
   copy(o->gamma, v.gamma, m * sizeof(double));
-  // vectors are interleaved on the device and land in the caller's arrays as
-  // they are (a host loop over 723,024 contacts took about as long as their
-  // transfer), in pieces through the packed records of the detection that
-  // found the contacts: the next detection writes those anew, so the download
-  // needs no memory of its own
   const double* trip[4][3] = {{v.nx, v.ny, v.nz}, {v.rix, v.riy, v.riz}, {v.rjx, v.rjy, v.rjz}, {v.cpx, v.cpy, v.cpz}};
   double* outs[4] = {o->normal, o->r_i, o->r_j, o->contact_point};
-  const size_t piece = ctx->pk.cap / 3;
   for (int f = 0; f < 4; ++f) {
     if (!outs[f]) continue;
     for (size_t k = 0; !e && k < m; k += piece) {
       const size_t count = m - k < piece ? m - k : piece;
-      e = interleave3(ctx, trip[f][0] + k, trip[f][1] + k, trip[f][2] + k, count, ctx->pk.p);
-      copy(outs[f] + 3 * k, ctx->pk.p, 3 * count * sizeof(double));
+      e = interleave3(ctx, trip[f][0] + k, trip[f][1] + k, trip[f][2] + k, count, scratch);
+      copy(outs[f] + 3 * k, scratch, 3 * count * sizeof(double));
     }
   }
   const cudaError_t done = cudaStreamSynchronize(s);

@@ -85,9 +85,11 @@ struct pcc_ctx {
   size_t ncons = 0;
   pcc::ConsBufs cons;
 
+  pcc::DevBuf<double> interleaved;  // vectors of the contacts on their way to the host
+
   // detection scratch
   pcc::DevBuf<int> bin_of, bin_cnt, bin_off, bin_raw, bin_cells, cand_cnt, cand_off;
-  pcc::DevBuf<double> pk;  // packed per-cell geometry in bin order (between detections: scratch of the contact download)
+  pcc::DevBuf<double> pk;  // packed per-cell geometry in bin order (between detections: spare scratch of the contact download)
   pcc::DevBuf<int> ghost;
   bool box_known = false;  // radius bounds the centres of the resident cells
   bool flat = true;        // no cell left the plane z = 0 since the upload

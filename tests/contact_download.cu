@@ -3,15 +3,17 @@
 // makes replaced by host stand-ins that copy at once, count what is still in
 // flight and fail on request.  Whatever fails, the call must return an error
 // with nothing in flight; if nothing fails, every array must arrive whole, also
-// when the vectors go through several pieces.  Prints "ok <cases>" or the
-// first failure.
+// on a device too full for a scratch of its own, where the vectors go through
+// several pieces.  Prints "ok <cases>" or the first failure.
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
 static int g_calls, g_fail_at, g_in_flight;  // g_fail_at: the call that fails, counted from 1 (0: none)
+static bool g_full;  // no device memory is left
 static bool fails() { return ++g_calls == g_fail_at; }
 
 static cudaError_t stand_in_copy(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t) {
@@ -25,8 +27,10 @@ static cudaError_t stand_in_sync(cudaStream_t) {
   return fails() ? cudaErrorUnknown : cudaSuccess;
 }
 template <class T>
-static cudaError_t stand_in_malloc(T**, size_t, cudaStream_t) {
-  return cudaErrorMemoryAllocation;  // the device is full
+static cudaError_t stand_in_malloc(T** p, size_t bytes, cudaStream_t) {
+  if (g_full) return cudaErrorMemoryAllocation;
+  *p = static_cast<T*>(malloc(bytes));  // kept: the program ends soon
+  return cudaSuccess;
 }
 
 #define cudaMemcpyAsync stand_in_copy
@@ -48,7 +52,7 @@ cudaError_t interleave3(pcc_ctx*, const double* x, const double* y, const double
 
 int main() {
   long long cases = 0;
-  const size_t sizes[] = {1, 2, 63, 64, 65, 1000}, rooms[] = {3, 64, 300, 3000, 5000};
+  const size_t sizes[] = {1, 2, 63, 64, 65, 1000}, rooms[] = {0, 3, 64, 300, 3000, 5000};  // 0: the device has room
   for (size_t m : sizes) {
     for (size_t room : rooms) {
       pcc_ctx* ctx = new pcc_ctx();  // kept: its buffers are not device memory
@@ -71,6 +75,7 @@ int main() {
         ib[q]->p = ids[q].data();
         ib[q]->cap = m;
       }
+      g_full = room != 0;
       std::vector<double> scratch(room);
       ctx->pk.p = scratch.data();
       ctx->pk.cap = room;
